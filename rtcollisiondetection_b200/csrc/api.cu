@@ -400,8 +400,8 @@ struct rtcd_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     DevBuf err;
-    DevBuf knn_w2;  // squared neighbour-search weights
-    std::mutex mu;  // guards knn_w2
+    cudaEvent_t default_done = nullptr;  // orders a call after the default stream's work
+    std::mutex mu;                       // guards default_done
 };
 
 struct rtcd_robot {
@@ -641,6 +641,7 @@ rtcd_status rtcd_context_create(int device, rtcd_ctx** out) {
             delete c;
             cuda_check(e, "cudaStreamCreate");
         }
+        cuda_check(cudaEventCreateWithFlags(&c->default_done, cudaEventDisableTiming), "cudaEventCreate");
         c->err.ensure(4);
         cuda_check(cudaMemset(c->err.p, 0, 4), "memset");
         *out = c;
@@ -653,6 +654,7 @@ rtcd_status rtcd_context_destroy(rtcd_ctx* ctx) {
         DeviceScope ds(ctx->device);
         cudaStreamSynchronize(ctx->stream);
         cudaStreamDestroy(ctx->stream);
+        cudaEventDestroy(ctx->default_done);
         ctx->err.release();
         delete ctx;
     });
@@ -2040,13 +2042,13 @@ rtcd_status rtcd_knn(rtcd_ctx* ctx, const float* points_dev, uint32_t n, uint32_
         RTCD_REQUIRE(k >= 1 && k <= kKnnMaxK, "k must be 1..32");
         DeviceScope ds(ctx->device);
         cudaStream_t s = stream ? (cudaStream_t) stream : ctx->stream;
-        std::lock_guard<std::mutex> lk(ctx->mu);
         float w2[kKnnMaxDim];
         for (uint32_t d = 0; d < dim; ++d) w2[d] = weights ? weights[d] * weights[d] : 1.0f;
-        ctx->knn_w2.ensure(sizeof(w2));
-        cuda_check(cudaStreamSynchronize(s), "knn weights");  // the previous call's kernel may still read them
-        cuda_check(cudaMemcpy(ctx->knn_w2.p, w2, dim * sizeof(float), cudaMemcpyHostToDevice), "knn weights");
-        launch_knn(points_dev, n, dim, ctx->knn_w2.as<float>(), k, mask_dev, idx_dev, dist_dev, s);
+        // points and outputs prepared on the default stream are ready before the search starts
+        std::lock_guard<std::mutex> lk(ctx->mu);
+        cuda_check(cudaEventRecord(ctx->default_done, cudaStreamLegacy), "event");
+        cuda_check(cudaStreamWaitEvent(s, ctx->default_done, 0), "event");
+        launch_knn(points_dev, n, dim, w2, k, mask_dev, idx_dev, dist_dev, s);
     });
 }
 

@@ -218,7 +218,8 @@ void launch_probe_sweep(bool quad, const float* d_seg, const float* d_piece, uin
 // planner side (planner.cu)
 constexpr uint32_t kKnnMaxK = 32;
 constexpr uint32_t kKnnMaxDim = 16;
-void launch_knn(const float* pts, uint32_t n, uint32_t dim, const float* w2_dev, uint32_t k, const uint8_t* mask,
+// w2: the squared weights (host).
+void launch_knn(const float* pts, uint32_t n, uint32_t dim, const float* w2, uint32_t k, const uint8_t* mask,
                 uint32_t* idx, float* dist, cudaStream_t s);
 void launch_interp_edges(const float* nodes, uint32_t n_nodes, uint32_t dof, const uint32_t* edges, uint32_t n_edges,
                          uint32_t n_wp, float* q, uint32_t* err, cudaStream_t s);

@@ -8,9 +8,8 @@
 // excluded, a partial insertion sort, square roots), and turns each edge
 // into a straight line of evenly spaced configurations that it checks as a
 // trajectory (RTCD/Utils/Test/poseUtils.h:115-141).  Here the neighbour search
-// is one warp per query (each lane keeps its own K best, the warp merges
-// them), and an edge check interpolates the edges on the device and runs the
-// detector over them in one call.
+// is one kernel, a lane per query (k_knn), and an edge check interpolates the
+// edges on the device and runs the detector over them in one call.
 #include <algorithm>
 #include <cfloat>
 #include <vector>
@@ -20,69 +19,274 @@
 
 namespace rtcd {
 
-constexpr int kKnnWarps = 4;
+// Squared axis weights, a kernel parameter (unused axes zero).
+struct KnnWeights {
+    float w2[kKnnMaxDim];
+};
 
-// One warp per query point.  Each lane scans every 32nd reference point and
-// keeps its own K smallest (distance, index) pairs, ordered; the warp then
-// pops the smallest head K times.  Pairs compare by distance, then by index,
-// which is the order the reference's insertion sort settles ties in.
-__global__ void __launch_bounds__(kKnnWarps * 32) k_knn(const float* __restrict__ pts, uint32_t n, uint32_t dim,
-                                                         const float* __restrict__ w2, uint32_t k,
-                                                         const uint8_t* __restrict__ mask, uint32_t* __restrict__ idx,
-                                                         float* __restrict__ dist) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t q = blockIdx.x * kKnnWarps + (threadIdx.x >> 5);
-    if (q >= n) return;  // warp-uniform
-    float qp[kKnnMaxDim], ww[kKnnMaxDim];
-    for (uint32_t d = 0; d < dim; ++d) {
-        qp[d] = pts[(size_t) q * dim + d];
-        ww[d] = w2[d];
+constexpr int kKnnBuf = 8;    // points a lane lets wait before the warp inserts them
+constexpr int kKnnStep = 4;   // reference points per inner step
+
+// Two FP32 operations in one instruction, each half rounded as the scalar one.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The smaller of two, NaN when either is.
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// Shared memory of one warp: the lanes' ordered lists [k][32], their waiting
+// points [kKnnBuf][32] and the warp's 32 reference points [dim + 1][32].
+__host__ __device__ constexpr size_t knn_warp_bytes(uint32_t k, uint32_t dim) {
+    return 256ull * k + 128ull * kKnnBuf + 128ull * (dim + 1);
+}
+
+// A block answers 32 queries, one per lane; its warps share the queries and
+// split the reference points.  A warp stages 32 points at a time in shared
+// memory and every lane reads each of them (a broadcast).
+//
+// A point r is passed over when a lower bound of its distance is above the
+// lane's bound: with N(x) = sum w2 x^2 the squared distance is N(q) + N(r) -
+// 2 sum w2 q r, one multiply-add per axis instead of the three operations of
+// w2 (r - q)^2, and both N are shrunk by kKnnSlack(dim), which covers every
+// rounding of either form (relative to N(q) + N(r), with u = 2^-24: the norms
+// (dim + 2) u, the sum 2 (dim + 1) u, the bound's difference u, and, while the
+// bound is at most 4 (N(q) + N(r)), 4 (dim + 5) u from the direct form's own
+// rounding; a larger bound lets the point through by itself).  What is
+// let through waits in a small buffer; when a lane's is full the warp computes
+// the distances themselves, in the direct form, and inserts them, so the lanes'
+// insertions run together.  Norms above 1e37 and NaNs make the test let
+// everything through.
+//
+// The bound of a query is the smaller of its warp's k-th distance and the
+// largest, over the block's warps, of the distance in place ceil(k / warps):
+// each warp holds that many pairs within it, so all together hold k.  (The
+// k-th distance of one warp's share of the points alone lets several times as
+// many pairs through.)  A sample of the points gives the first bound.  The
+// warps' lists are merged at the end.  Pairs are 64-bit keys (distance bits,
+// index): distances are never negative, so key order is by distance, then by
+// index, which is the order the reference's insertion sort settles ties in; a
+// NaN sorts after the empty entry and never enters.
+//
+// Bound by instruction issue.  20,000 points of 7 axes, k = 10: one warp per
+// query with a list per lane in local memory (about 1,300 divergent insertion
+// steps per query) 4,406 us; the direct form for every pair here 557 us; this
+// form 452 us.
+__host__ __device__ constexpr float knn_slack(int dim) { return (float) (8 * dim + 32) / 16777216.0f; }
+
+template <int DIM>
+__global__ void __launch_bounds__(1024) k_knn(const float* __restrict__ pts, uint32_t n, const KnnWeights wt, uint32_t k,
+                                              const uint8_t* __restrict__ mask, uint32_t* __restrict__ idx,
+                                              float* __restrict__ dist) {
+    extern __shared__ __align__(16) uint64_t s_dyn[];
+    __shared__ float s_rank[32][32];  // [warp][query] distance of the warp's entry number `share`
+    __shared__ float s_q[DIM][32];    // the queries
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const size_t stride = knn_warp_bytes(k, DIM) / 8;
+    uint64_t* list = s_dyn + stride * warp;
+    uint32_t* buf = reinterpret_cast<uint32_t*>(list + 32 * k);
+    float* tile = reinterpret_cast<float*>(buf + 32 * kKnnBuf);
+    const uint64_t empty = ((uint64_t) __float_as_uint(FLT_MAX) << 32) | 0xFFFFFFFFu;
+    const float nan = __uint_as_float(0x7FC00000u), inf = __uint_as_float(0x7F800000u);
+    constexpr float kKeep = 1.0f - knn_slack(DIM), kMostNorm = 1e37f;
+
+    const uint32_t q = blockIdx.x * 32 + lane;
+    const bool live = q < n && !(mask && mask[q]);
+    float norm_q = 0.f;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const float v = live ? pts[(size_t) q * DIM + d] : 0.f;
+        if (warp == 0) s_q[d][lane] = v;
+        norm_q = fmaf(v * v, wt.w2[d], norm_q);
     }
-    float bd[kKnnMaxK];
-    uint32_t bi[kKnnMaxK];
-    for (uint32_t j = 0; j < k; ++j) {
-        bd[j] = FLT_MAX;
-        bi[j] = 0xFFFFFFFFu;
+    uint64_t m2wq[DIM];  // -2 w2 q, twice each
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const float v = live ? pts[(size_t) q * DIM + d] : 0.f;
+        const float m = norm_q <= kMostNorm ? -2.f * wt.w2[d] * v : nan;
+        m2wq[d] = pack2(m, m);
     }
-    const bool qmasked = mask && mask[q];
-    for (uint32_t r = lane; r < n; r += 32) {
-        if (r == q || qmasked || (mask && mask[r])) continue;  // not a candidate
-        float s = 0.f;
-        for (uint32_t d = 0; d < dim; ++d) {
-            const float t = pts[(size_t) r * dim + d] - qp[d];
-            s += t * t * ww[d];
+    norm_q *= kKeep;
+    for (uint32_t j = 0; j < k; ++j) list[j * 32 + lane] = empty;
+    __syncthreads();
+
+    const uint32_t share = (k + warps - 1) / warps;
+    float bound = FLT_MAX, limit = live ? FLT_MAX : -inf;  // limit: the bound less the query's norm
+    int held = 0;
+    auto set_bound = [&](float b) {
+        if (b < bound) {
+            bound = b;
+            limit = live ? b - norm_q + 1e-36f : -inf;  // 1e-36: above the roundings of subnormal terms
         }
-        // insert into this lane's ordered list when better than its last entry
-        if (s < bd[k - 1] || (s == bd[k - 1] && r < bi[k - 1])) {
-            int j = (int) k - 1;
-            while (j > 0 && (s < bd[j - 1] || (s == bd[j - 1] && r < bi[j - 1]))) {
-                bd[j] = bd[j - 1];
-                bi[j] = bi[j - 1];
-                --j;
+    };
+    auto tighten = [&] {
+        float joint = 0.f;
+        for (int w = 0; w < warps; ++w) joint = fmaxf(joint, *(volatile float*) &s_rank[w][lane]);
+        set_bound(joint);
+    };
+    float rank = FLT_MAX;
+    auto publish = [&](float v) {
+        rank = fminf(rank, v);
+        *(volatile float*) &s_rank[warp][lane] = rank;
+    };
+    auto insert_held = [&] {
+        for (int e = 0; e < held; ++e) {
+            const uint32_t r = buf[e * 32 + lane];
+            if (!live || r == q || r >= n || (mask && mask[r])) continue;
+            float s = 0.f;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                const float t = __fsub_rn(__ldg(pts + (size_t) r * DIM + d), s_q[d][lane]);
+                s = __fmaf_rn(__fmul_rn(t, t), wt.w2[d], s);
             }
-            bd[j] = s;
-            bi[j] = r;
+            const uint64_t key = ((uint64_t) __float_as_uint(s) << 32) | r;
+            // one pass over the list: every entry is read whatever the others hold, so the reads
+            // overlap (a search from the end waits for each entry before the next)
+            uint64_t cur = list[(k - 1) * 32 + lane];
+            bool below = key < cur;
+            if (!below) continue;
+#pragma unroll 4
+            for (int j = (int) k - 1; j > 0; --j) {
+                const uint64_t up = list[(j - 1) * 32 + lane];
+                const bool next_below = key < up;
+                list[j * 32 + lane] = next_below ? up : (below ? key : cur);
+                cur = up;
+                below = next_below;
+            }
+            list[lane] = below ? key : cur;
+        }
+        held = 0;
+        set_bound(__uint_as_float((uint32_t) (list[(k - 1) * 32 + lane] >> 32)));
+        publish(__uint_as_float((uint32_t) (list[(share - 1) * 32 + lane] >> 32)));
+    };
+
+    // the warps take the 32-point tiles in turn; a lane loads one point of a tile
+    const uint32_t tiles = (n + 31) / 32;
+    float next[DIM];
+    bool next_on;
+    auto load_tile = [&](uint32_t t) {
+        const uint32_t r = t * 32 + lane;
+        next_on = t < tiles && r < n && !(mask && mask[r]);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) next[d] = next_on ? __ldg(pts + (size_t) r * DIM + d) : 0.f;
+    };
+    auto store_tile = [&] {  // the points, then their shrunken norms (infinite: no point)
+        float norm = 0.f;
+        __syncwarp();
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            tile[d * 32 + lane] = next[d];
+            norm = fmaf(next[d] * next[d], wt.w2[d], norm);
+        }
+        tile[DIM * 32 + lane] = !next_on ? inf : norm <= kMostNorm ? norm * kKeep : nan;
+        __syncwarp();
+    };
+
+    // the lower bounds, less the query's norm, of points r0 .. r0 + 3 of the tile
+    auto lower = [&](int r0, float* s, float* norm) {
+        const ulonglong2 nr = *reinterpret_cast<const ulonglong2*>(tile + DIM * 32 + r0);
+        uint64_t s01 = nr.x, s23 = nr.y;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(tile + d * 32 + r0);
+            s01 = fma2(p.x, m2wq[d], s01);
+            s23 = fma2(p.y, m2wq[d], s23);
+        }
+        const float2 a = unpack2(s01), b = unpack2(s23), c = unpack2(nr.x), d = unpack2(nr.y);
+        s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
+        norm[0] = c.x; norm[1] = c.y; norm[2] = d.x; norm[3] = d.y;
+    };
+
+    // a first bound from a sample of the warp's points: upper bounds of its four smallest distances
+    // (three slacks above the lower ones)
+    {
+        constexpr float kUp = 3.0f * knn_slack(DIM);
+        const uint32_t mine = (tiles + warps - 1) / warps;
+        const uint32_t sample = max(mine / 16, 1u);
+        float m[4] = {FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX};
+        load_tile(warp);
+        for (uint32_t i = 0; i < sample; ++i) {
+            const uint32_t t = warp + i * warps;
+            store_tile();
+            load_tile(t + warps);
+#pragma unroll 2
+            for (int r0 = 0; r0 < 32; r0 += kKnnStep) {
+                float s[kKnnStep], norm[kKnnStep];
+                lower(r0, s, norm);
+#pragma unroll
+                for (int j = 0; j < kKnnStep; ++j) {
+                    float v = fminf(fmaf(kUp, norm[j], s[j]), FLT_MAX);  // a NaN counts as FLT_MAX
+                    if (t * 32 + r0 + j == q) v = FLT_MAX;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float up = fmaxf(m[c], v);
+                        m[c] = fminf(m[c], v);
+                        v = up;
+                    }
+                }
+            }
+        }
+        const float mth = share == 1 ? m[0] : share == 2 ? m[1] : share == 3 ? m[2] : share == 4 ? m[3] : FLT_MAX;
+        publish(fminf(fmaxf(mth + fmaf(kUp, norm_q, norm_q), 0.f) + 1e-36f, FLT_MAX));
+    }
+    __syncthreads();
+
+    load_tile(warp);
+    for (uint32_t t = warp; t < tiles; t += warps) {
+        store_tile();
+        load_tile(t + warps);
+        tighten();
+#pragma unroll 2
+        for (int r0 = 0; r0 < 32; r0 += kKnnStep) {
+            float s[kKnnStep], norm[kKnnStep];
+            lower(r0, s, norm);
+            if (__any_sync(0xffffffffu, !(min_nan(min_nan(s[0], s[1]), min_nan(s[2], s[3])) > limit))) {
+#pragma unroll
+                for (int j = 0; j < kKnnStep; ++j)
+                    if (!(s[j] > limit)) buf[32 * held++ + lane] = t * 32 + r0 + j;
+                if (__any_sync(0xffffffffu, held > kKnnBuf - kKnnStep)) {
+                    insert_held();
+                    tighten();
+                }
+            }
         }
     }
-    // merge: k rounds of a warp arg-min over the lanes' heads
+    insert_held();
+    __syncthreads();
+
+    // merge: `warps` neighbouring lanes (a power of two) per query, one list each
+    const int group = threadIdx.x / warps, member = threadIdx.x % warps;  // blockDim.x / warps = 32 queries
+    const uint64_t* mine = s_dyn + stride * member + group;
+    const uint32_t out_q = blockIdx.x * 32 + group;
     uint32_t head = 0;
     for (uint32_t out = 0; out < k; ++out) {
-        float v = head < k ? bd[head] : FLT_MAX;
-        uint32_t i = head < k ? bi[head] : 0xFFFFFFFFu;
-        float bv = v;
-        uint32_t bidx = i;
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const uint32_t oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-            if (ov < bv || (ov == bv && oi < bidx)) {
-                bv = ov;
-                bidx = oi;
-            }
+        const uint64_t top = head < k ? mine[head * 32] : empty;
+        uint64_t best = top;
+        for (int o = warps >> 1; o > 0; o >>= 1) {
+            const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
+            best = other < best ? other : best;
         }
-        if (v == bv && i == bidx && head < k) ++head;  // the winning lane advances (indices are unique)
-        if (lane == 0) {
-            idx[(size_t) q * k + out] = bidx;
-            dist[(size_t) q * k + out] = bv < FLT_MAX ? sqrtf(bv) : FLT_MAX;
+        if (top == best && head < k) ++head;  // keys are unique, so one list advances
+        if (member == 0 && out_q < n) {
+            const float v = __uint_as_float((uint32_t) (best >> 32));
+            idx[(size_t) out_q * k + out] = (uint32_t) best;
+            dist[(size_t) out_q * k + out] = v < FLT_MAX ? sqrtf(v) : FLT_MAX;
         }
     }
 }
@@ -118,11 +322,39 @@ __global__ void k_or_rows(const uint8_t* __restrict__ pose_flags, uint32_t n_edg
     flags[e] = f;
 }
 
-void launch_knn(const float* pts, uint32_t n, uint32_t dim, const float* w2_dev, uint32_t k, const uint8_t* mask,
+// Warps per block, a power of two: eight fill the SMs once there are two blocks
+// of 32 queries for each; with fewer blocks the points are split over more
+// warps, as far as every warp has a tile of them and the shared memory of a
+// block allows.
+template <int DIM>
+static void launch_knn_dim(const float* pts, uint32_t n, const KnnWeights& w, uint32_t k, const uint8_t* mask,
+                           uint32_t* idx, float* dist, cudaStream_t s) {
+    constexpr size_t kMost = 200 * 1024;
+    const uint32_t blocks = (n + 31) / 32;
+    uint32_t warps = 1;
+    while (warps < 32 && 2 * warps <= blocks && (warps < 8 || blocks * warps < 16u * (uint32_t) device_sm_count()) &&
+           2 * warps * knn_warp_bytes(k, DIM) <= kMost)
+        warps *= 2;
+    const size_t smem = warps * knn_warp_bytes(k, DIM);
+    if (smem > 47 * 1024)
+        cuda_check(cudaFuncSetAttribute(k_knn<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kMost), "k_knn");
+    k_knn<DIM><<<blocks, warps * 32, smem, s>>>(pts, n, w, k, mask, idx, dist);
+    cuda_check(cudaGetLastError(), "k_knn");
+}
+
+template <int DIM = 1>
+static void knn_dispatch(uint32_t dim, const float* pts, uint32_t n, const KnnWeights& w, uint32_t k,
+                         const uint8_t* mask, uint32_t* idx, float* dist, cudaStream_t s) {
+    if (dim == (uint32_t) DIM) return launch_knn_dim<DIM>(pts, n, w, k, mask, idx, dist, s);
+    if constexpr (DIM < (int) kKnnMaxDim) knn_dispatch<DIM + 1>(dim, pts, n, w, k, mask, idx, dist, s);
+}
+
+void launch_knn(const float* pts, uint32_t n, uint32_t dim, const float* w2, uint32_t k, const uint8_t* mask,
                 uint32_t* idx, float* dist, cudaStream_t s) {
     if (!n) return;
-    k_knn<<<(n + kKnnWarps - 1) / kKnnWarps, kKnnWarps * 32, 0, s>>>(pts, n, dim, w2_dev, k, mask, idx, dist);
-    cuda_check(cudaGetLastError(), "k_knn");
+    KnnWeights w{};
+    for (uint32_t d = 0; d < dim; ++d) w.w2[d] = w2[d];
+    knn_dispatch(dim, pts, n, w, k, mask, idx, dist, s);
 }
 
 void launch_interp_edges(const float* nodes, uint32_t n_nodes, uint32_t dof, const uint32_t* edges, uint32_t n_edges,
