@@ -826,7 +826,7 @@ def main():
     if sweep:
         span = ('k_sweep_traj' if st['path_flags'] & 1 else 'k_sweep') + ' + k_sweep_heavy x 2 (heavy, split)'
     elif form in (0, 3, 4):
-        span = 'k_stage_ab + k_subtree x 2 + k_stage_b (deferred) + k_stage_b_heavy + k_discrete (overflow)'
+        span = 'k_query'
     else:
         span = 'k_stage_a + k_stage_b%s + k_stage_b_heavy + k_discrete (overflow)' % ('_packet' if form == 2 else '')
     traffic = None

@@ -133,32 +133,28 @@ typedef struct {
     int32_t stream_priority;         /* priority of the detector's own stream (CUDA convention: lower = higher) */
     uint32_t residency_percent;      /* share of each SM its persistent kernels may hold (room for other
                                         launches to run alongside); 0 = 100 */
-    uint32_t light_steps;            /* node + leaf visits one lane spends on a unit of traversal work (a
-                                        discrete (link item, scene primitive) candidate, a sweep (piece,
-                                        sphere) unit) before a whole warp takes it over; 0 = 32 (16 for
-                                        the sweeps), 0xFFFFFFFF = never */
-    uint32_t stage_b_form;           /* discrete stage B: 1 = one lane per candidate, 2 = 32-candidate packets
-                                        that share each link-BVH node load, 3 = stages A and B fused in one
-                                        warp per item (an item stops generating candidates once its pose
-                                        is hit), 4 = 3 with packet descents of the link tree; 0 = 3 (the
-                                        autotuner tries all four).  Sweeps: 1 = the light pass's lanes descend
-                                        the binary edge tree, any other value the 4-wide one (when the
-                                        scene's is shallow enough for a lane stack; the autotuner tries
-                                        both) */
-    uint32_t stage_b_chunk;          /* discrete stage B: consecutive candidates one lane takes in order (lanes
+    uint32_t light_steps;            /* node + leaf visits one lane spends on a unit of traversal work (a sweep
+                                        (piece, sphere) unit; for discrete forms 1 and 2 a (link item, scene
+                                        primitive) candidate) before a whole warp takes it over; 0 = 16 for
+                                        the sweeps, 32 for the discrete forms, 0xFFFFFFFF = never */
+    uint32_t stage_b_form;           /* discrete traversal: 0 (also 3 and 4) = the query kernel: one launch, one warp
+                                        per item or part of one, work shared between the warps as it runs;
+                                        the other forms write every candidate to memory and descend the link
+                                        trees in a second kernel: 1 = one lane per candidate, 2 =
+                                        32-candidate packets that share each link-BVH node load.  Sweeps: 1 =
+                                        the light pass's lanes descend the binary edge tree, any other value
+                                        the 4-wide one (when the scene's is shallow enough for a lane stack).
+                                        The autotuner tries them */
+    uint32_t stage_b_chunk;          /* discrete forms 1 and 2: consecutive candidates one lane takes in order (lanes
                                         form) or 32-candidate groups one warp takes (packets), so a pose's
-                                        candidates spread over few workers that stop at its first hit; for
-                                        the fused forms, the stage-B steps (32 candidates each) an item runs
-                                        in its warp before its further candidates go to a one-lane pass over
-                                        the whole GPU; 0 = 64 lanes / 4 packets / 8 steps; at most 4096 */
+                                        candidates spread over few workers that stop at its first hit;
+                                        0 = 64 lanes / 4 packets; at most 4096; without effect on form 0 */
     uint32_t plain_streams;          /* streams of the plain path, each driven by its own host thread; frames go to
                                         them round-robin and the call waits for every group of plain_streams
                                         frames (upstream NSTREAM = 4 and its thread pool,
                                         RTCD/CollisionDetector/CollisionDetector.h:396-433); 0 = 4, at most 16 */
-    uint32_t top_nodes_shared;       /* discrete fused form: wide scene-tree nodes (breadth-first from the root: its
-                                        top levels) each block copies to shared memory and its descents read
-                                        there; 0 = none, at most 256 (the autotuner tries 0 and 85, the first
-                                        four levels) */
+    uint32_t top_nodes_shared;       /* accepted up to 256, without effect (the query kernel reads the scene tree's
+                                        top levels through L1) */
     uint32_t sweep_unstaged;         /* sweeps: 0 = the light pass stages each trajectory's FK (and quadratic fit)
                                         in shared memory when the batch's longest trajectory fits and the batch
                                         has at least four trajectories per resident block; 1 = sphere centres
@@ -295,9 +291,9 @@ RTCD_API rtcd_status rtcd_sync(rtcd_detector* det, void* stream);
  * host for sweeps) with every traversal launch shape - 64, 128 and 256
  * threads per block, each at a quarter, half and all of the blocks per SM
  * that fit; then light-pass budgets (light_steps) of the default, 16, 32 and
- * 64 visits; then, for the discrete kinds, the four stage B forms at chunk
- * lengths from 1 to 256 candidates and the shared-memory top levels, for the
- * sweeps the binary and the 4-wide edge tree, staged or unstaged centres and
+ * 64 visits; then, for the discrete kinds, the query kernel and the two
+ * wavefront forms at chunk lengths from 1 to 256 candidates, for the sweeps
+ * the binary and the 4-wide edge tree, staged or unstaged centres and
  * grouped or single trajectories; then the launch shapes again - rounds of
  * this coordinate descent until one changes nothing (at most three; sweeps
  * are timed with segment flags on)

@@ -408,6 +408,7 @@ struct rtcd_robot {
     rtcd_ctx* ctx = nullptr;
     RobotDev dev{};
     GroupedBvh tri, edge;
+    DevBuf tri_wide, edge_wide;  // 4-wide copies of the link trees
     DevBuf verts, tris, edges, spheres, sphere_link;
     std::vector<uint32_t> edge_off;
     uint32_t dof = 0;
@@ -517,7 +518,8 @@ struct rtcd_detector {
     uint32_t blocks = 0;
     // discrete workspace
     DevBuf q, T, mask, items, count, pose_hit, counts, edge_bits, flags, seg_flags, work, err, stats, contain;
-    DevBuf cand, item_overflow, overflow_items, wave_counts, sub;  // wavefront traversal
+    DevBuf query;  // the query kernel's queue: counters and slots
+    DevBuf cand, item_overflow, overflow_items, wave_counts;  // wavefront traversal (stage_b_form 1, 2)
     uint32_t blocks_a = 0, blocks_b = 0, blocks_a_full = 0;
     uint32_t threads = 128;  // traversal launch shape (stage B / sweep kernel)
     ScanScratch scan;
@@ -741,7 +743,23 @@ rtcd_status rtcd_robot_create(rtcd_ctx* ctx, const rtcd_robot_desc* d, rtcd_robo
         r->dev.tri_prims = r->tri.prims.as<float4>();
         r->dev.edge_nodes = r->edge.nodes.as<float4>();
         r->dev.edge_prims = r->edge.prims.as<float4>();
+        const auto link_nodes = [&](const std::vector<uint32_t>& off) {
+            uint32_t n = 0;
+            for (uint32_t l = 0; l < L; ++l) n += off[l + 1] > off[l] ? off[l + 1] - off[l] - 1 : 0;
+            return n;
+        };
+        std::vector<uint32_t> tri_wide_roots, edge_wide_roots;
+        r->dev.tri_wide_depth =
+            build_wide_forest(r->dev.tri_nodes, link_nodes(toff), r->tri.roots, tri_wide_roots, r->tri_wide, s).depth;
+        r->dev.edge_wide_depth =
+            build_wide_forest(r->dev.edge_nodes, link_nodes(eoff), r->edge.roots, edge_wide_roots, r->edge_wide, s).depth;
+        // pairs hold a link reference beside a candidate's tag (wide.cuh)
+        r->dev.pair_refs = std::max(toff[L], eoff[L]) < (1u << 27) ? 1u : 0u;
+        r->dev.tri_wide = r->tri_wide.as<float4>();
+        r->dev.edge_wide = r->edge_wide.as<float4>();
         for (uint32_t l = 0; l < (uint32_t) kMaxLinks; ++l) {
+            r->dev.tri_wide_root[l] = l < L ? tri_wide_roots[l] : kNone;
+            r->dev.edge_wide_root[l] = l < L ? edge_wide_roots[l] : kNone;
             r->dev.tri_root[l] = l < L ? r->tri.roots[l] : kNone;
             r->dev.edge_root[l] = l < L ? r->edge.roots[l] : kNone;
         }
@@ -858,14 +876,13 @@ rtcd_status rtcd_scene_create(rtcd_ctx* ctx, const float* verts, uint32_t n_vert
         dv.tri_wide_root = wt.root;
         dv.edge_wide = sc->edge_wide.as<float4>();
         dv.edge_wide_root = we.root;
-        dv.wide_front = wide_frontier(std::max(wt.depth, we.depth));
         upload(sc->tri_cut, wt.cut.data(), wt.cut.size(), s);
         upload(sc->edge_cut, we.cut.data(), we.cut.size(), s);
         dv.tri_cut = sc->tri_cut.as<float4>();
         dv.edge_cut = sc->edge_cut.as<float4>();
         dv.n_tri_cut = (uint32_t) wt.cut.size() / 2;
-        dv.n_tri_wide = wt.nodes;
-        dv.n_edge_wide = we.nodes;
+        dv.tri_wide_depth = wt.depth;
+        dv.edge_wide_depth = we.depth;
         dv.n_edge_cut = (uint32_t) we.cut.size() / 2;
         // a depth-first lane descent keeps at most 3 siblings per level plus the last node's 4 children
         dv.edge_wide_lane = (kWide - 1) * we.depth + kWide <= (uint32_t) kStack ? 1u : 0u;
@@ -1033,9 +1050,8 @@ const SceneDev& scene_loop(rtcd_scene* sc) {
     dv.edge_wide_root = w.root;
     dv.edge_cut = sc->loop_cut.as<float4>();
     dv.n_edge_cut = (uint32_t) w.cut.size() / 2;
-    dv.n_edge_wide = w.nodes;
     dv.edge_wide_lane = (kWide - 1) * w.depth + kWide <= (uint32_t) kStack ? 1u : 0u;
-    dv.wide_front = std::max(dv.wide_front, wide_frontier(w.depth));
+    dv.edge_wide_depth = w.depth;
     cuda_check(cudaStreamSynchronize(s), "loop-edge trees");
     sc->dev_loop = dv;
     sc->loop_built = true;
@@ -1175,36 +1191,50 @@ static void traverse(rtcd_detector* d, bool r2o, const DiscreteArgs& A, uint32_t
                      uint32_t flags, cudaStream_t s, cudaEvent_t ev_first) {
     RobotDev& R = d->robot->dev;
     const uint32_t L = R.n_links;
+    const bool lane_form = d->cfg.stage_b_form == 1 || d->cfg.stage_b_form == 2;
+    const uint32_t share = d->cfg.residency_percent ? d->cfg.residency_percent : 100;
+    if (!(flags & RTCD_CHECK_FUSED) && !lane_form && R.pair_refs) {
+        const size_t query_bytes = 256 + sizeof(ulonglong2) * kQuerySlots;
+        d->query.ensure(query_bytes);
+        cuda_check(cudaMemsetAsync(d->query.p, 0, query_bytes, s), "memset");
+        uint8_t* base = d->query.as<uint8_t>();
+        QueryArgs Q{};
+        Q.d = A;
+        Q.d.work_counter = reinterpret_cast<uint32_t*>(base + 128);
+        Q.queue = reinterpret_cast<unsigned long long*>(base);
+        Q.live = reinterpret_cast<uint32_t*>(base + 64);
+        Q.slot = reinterpret_cast<ulonglong2*>(base + 256);
+        Q.slots = kQuerySlots;
+        launch_query(r2o, R, d->scene->dev, Q, (uint64_t) n * (L - R.first_link), share, plain ? blocks : 0xFFFFFFFFu, s);
+        if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
+        return;
+    }
     cuda_check(cudaMemsetAsync(d->work.p, 0, 8, s), "memset");
-    if (flags & RTCD_CHECK_FUSED) {
+    if ((flags & RTCD_CHECK_FUSED) || !lane_form) {
         launch_discrete(r2o, R, d->scene->dev, A, blocks, s);
         if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
         return;
     }
-    // stage A (+ B) -> heavy pass -> the thread-per-item kernel over items whose candidates overflowed
+    // stage A -> stage B -> heavy pass -> the thread-per-item kernel over items whose candidates overflowed
     const size_t items_max = (size_t) n * L;
     const uint32_t cap = (uint32_t) std::min<size_t>(std::max<size_t>(items_max * 128, 1u << 16), 1u << 26);
     d->cand.ensure(8ull * cap);
-    d->item_overflow.ensure(items_max + 4);  // marked a word at a time
+    d->item_overflow.ensure(items_max);
     d->overflow_items.ensure(4ull * items_max);
-    d->wave_counts.ensure(8 * 4);
-    cuda_check(cudaMemsetAsync(d->item_overflow.p, 0, items_max + 4, s), "memset");
-    cuda_check(cudaMemsetAsync(d->wave_counts.p, 0, 32, s), "memset");
-    // [0] candidates, [1] overflowed items, [2] fallback work, [3] heavy, [4..7] subtree pass
+    d->wave_counts.ensure(4 * 4);
+    cuda_check(cudaMemsetAsync(d->item_overflow.p, 0, items_max, s), "memset");
+    cuda_check(cudaMemsetAsync(d->wave_counts.p, 0, 16, s), "memset");
+    // [0] candidates, [1] overflowed items, [2] fallback work, [3] heavy
     uint32_t* wc = d->wave_counts.as<uint32_t>();
     WaveArgs W{};
     W.d = A;
-    W.top_nodes = d->cfg.top_nodes_shared;
     W.cand = d->cand.as<uint2>();
     W.cand_count = wc;
     W.cand_cap = cap;
     W.item_overflow = d->item_overflow.as<uint8_t>();
     W.overflow_items = d->overflow_items.as<uint32_t>();
     W.overflow_count = wc + 1;
-    const bool fused_form = d->cfg.stage_b_form == 0 || d->cfg.stage_b_form >= 3;
-    // lanes / packets: the chunk; fused forms: stage_b_chunk is the item's stage-B step budget
-    W.chunk = (!fused_form && d->cfg.stage_b_chunk) ? d->cfg.stage_b_chunk : (d->cfg.stage_b_form == 2 ? 4u : 64u);
-    W.item_steps = fused_form ? (d->cfg.stage_b_chunk ? d->cfg.stage_b_chunk : 8u) : 0xFFFFFFFFu;
+    W.chunk = d->cfg.stage_b_chunk ? d->cfg.stage_b_chunk : (d->cfg.stage_b_form == 2 ? 4u : 64u);
     W.light_steps = d->cfg.light_steps == 0xFFFFFFFFu ? 0u
                     : d->cfg.light_steps                ? d->cfg.light_steps
                                                               : 32u;
@@ -1216,32 +1246,12 @@ static void traverse(rtcd_detector* d, bool r2o, const DiscreteArgs& A, uint32_t
         W.heavy_count = wc + 3;
         W.heavy_work = d->work.as<uint32_t>() + 1;
     }
-    if (fused_form) {
-        const uint32_t scap = (uint32_t) std::min<size_t>(std::max<size_t>(items_max * 8, 1u << 16), 1u << 24);
-        d->sub.ensure(2 * 8ull * scap);
-        W.sub = d->sub.as<uint2>();
-        W.sub_cap = scap;
-        W.sub_count = wc + 4;
-    }
-    uint32_t ba = plain ? std::max<uint32_t>(1, blocks * kTravThreads / (kStageAWarps * 32)) : d->blocks_a;
-    const uint32_t share = d->cfg.residency_percent ? d->cfg.residency_percent : 100;
+    const uint32_t ba = plain ? std::max<uint32_t>(1, blocks * kTravThreads / (kStageAWarps * 32)) : d->blocks_a;
     WaveArgs W1 = W;  // the later passes count into bank 1
     W1.d.stats = A.stats + kStatBank;
-    if (fused_form) {
-        const bool packets = d->cfg.stage_b_form == 4;
-        const uint32_t full = stage_ab_blocks(r2o, packets, d->scene->dev);
-        launch_stage_ab(r2o, packets, R, d->scene->dev, W, plain ? std::min(ba, full) : std::max(1u, full * share / 100),
-                        s);
-        if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
-        // the rest of the crowded items' descents, the one-lane pass over the candidates they
-        // deferred, then the heavy pass
-        launch_subtree(r2o, R, d->scene->dev, W1, share, s);
-        launch_stage_b(r2o, R, d->scene->dev, W1, d->blocks_b, d->threads, share, false, s);
-    } else {
-        launch_stage_a(r2o, R, d->scene->dev, W, std::min(ba, d->blocks_a), s);
-        if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
-        launch_stage_b(r2o, R, d->scene->dev, W1, d->blocks_b, d->threads, share, d->cfg.stage_b_form == 2, s);
-    }
+    launch_stage_a(r2o, R, d->scene->dev, W, std::min(ba, d->blocks_a), s);
+    if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
+    launch_stage_b(r2o, R, d->scene->dev, W1, d->blocks_b, d->threads, share, d->cfg.stage_b_form == 2, s);
     DiscreteArgs F = A;
     F.stats = A.stats + kStatBank;
     F.items = d->overflow_items.as<uint32_t>();  // item words
@@ -1978,20 +1988,17 @@ rtcd_status rtcd_detector_autotune(rtcd_detector* d, const float* q_dev, const u
                 }
                 return;
             }
-            for (uint32_t form : {1u, 2u, 3u, 4u})
+            rtcd_config c = base;  // the query kernel, or the wavefront in lanes or packets
+            c.stage_b_form = c.stage_b_chunk = 0;
+            time_cfg(c);
+            for (uint32_t form : {1u, 2u})
                 for (uint32_t chunk : {1u, 16u, 64u, 256u}) {
-                    rtcd_config c = base;
+                    c = base;
                     c.stage_b_form = form;
-                    // lanes: candidates per lane; packets: groups per warp; fused: the item's
-                    // stage-B step budget (1, 4, 16, 64)
-                    c.stage_b_chunk = form == 2 ? std::max(1u, chunk / 16) : (form >= 3 ? std::max(1u, chunk / 4) : chunk);
+                    // lanes: candidates per lane; packets: groups per warp
+                    c.stage_b_chunk = form == 2 ? std::max(1u, chunk / 16) : chunk;
                     time_cfg(c);
                 }
-            if (best.stage_b_form == 0 || best.stage_b_form >= 3) {  // the fused form: top levels in shared memory
-                rtcd_config c = best;
-                c.top_nodes_shared = best.top_nodes_shared ? 0u : 85u;  // 1 + 4 + 16 + 64: the first four levels
-                time_cfg(c);
-            }
         };
         // rounds of descent over the three groups of settings until a round changes nothing (the
         // best light budget and stage-B form depend on the launch shape and back)

@@ -8,21 +8,22 @@
 // RT-core ray per edge (CCCuda.cu:56-77 ObsToRobot, CCRay.cu:74-116
 // RobotToObs).
 //
-// Here a work item is one (pose, link) pair that survived the cull.  One lane
-// owns one item and runs a two-stage query in a persistent loop:
-//   A. the link's world OBB descends the scene LBVH (triangles for
-//      RobotToObs, obstacle edges for ObsToRobot); each overlapping scene
-//      primitive becomes a candidate;
+// Here a work item is one (pose, link) pair that survived the cull, queried in
+// two stages:
+//   A. the link's world OBB descends the scene tree (triangles for RobotToObs,
+//      obstacle edges for ObsToRobot); each overlapping scene primitive becomes
+//      a candidate;
 //   B. the candidate is moved into the link frame (x_l = R^T (x - t)) and
-//      descends the static link LBVH (link edges for RobotToObs, link
-//      triangles for ObsToRobot); each overlapping pair gets the exact
-//      segment-triangle test.
+//      descends the static link tree (link edges for RobotToObs, link triangles
+//      for ObsToRobot); each overlapping pair gets the exact segment-triangle
+//      test.
 // Both sides are instanced - no per-batch acceleration structure is built -
 // and the result is the same predicate the upstream rays evaluate: some edge
-// of the source mesh crosses some triangle of the target mesh.  Lanes fetch new
-// items from a device counter as they finish (persistent threads), so uneven
-// items do not idle a warp.  Without counts, a pose stops as soon as one
-// of its items hits.
+// of the source mesh crosses some triangle of the target mesh.  k_query runs
+// both stages with a warp per item; k_discrete (RTCD_CHECK_FUSED) runs them
+// with a lane per item; k_stage_a and k_stage_b* (stage_b_form 1 and 2) write
+// the candidates to memory between them.  Without counts, a pose stops as soon
+// as one of its items hits.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -637,6 +638,50 @@ struct StageBCand {
     bool big;                 // R2O: a triangle large enough for the edge-axis node test
 };
 
+// Moves scene primitive `prim` into the frame of `link` (transform C.T) and
+// sets the candidate up: false when it does not reach the link's OBB.
+template <bool R2O>
+__device__ __forceinline__ bool cand_geometry(const RobotDev& R, const SceneDev& S, uint32_t link, uint32_t prim,
+                                              StageBCand& C) {
+    constexpr float kBoxTol = 2e-5f;
+    const float* lo = R.obb[link];
+    const f3 oc = mk(lo[0], lo[1], lo[2]);
+    const f3 u0 = mk(lo[6], lo[7], lo[8]), u1 = mk(lo[9], lo[10], lo[11]), u2 = mk(lo[12], lo[13], lo[14]);
+    const float4* __restrict__ wp = R2O ? S.tri_prims : S.edge_prims;
+    C.prim = prim;
+    C.c2 = C.cn = C.cinv = mk(0.f, 0.f, 0.f);
+    C.cw = 0.f;
+    C.big = false;
+    if (R2O) {
+        const float4* t = wp + 3ull * prim;
+        C.c0 = xf_inv(C.T, f3of(__ldg(t)));
+        C.c1 = xf_inv(C.T, f3of(__ldg(t + 1)));
+        C.c2 = xf_inv(C.T, f3of(__ldg(t + 2)));
+        C.cn = cross(C.c1 - C.c0, C.c2 - C.c0);
+        C.cw = dot(C.cn, C.c0);
+        const float rr = (lo[3] + kBoxTol) * fabsf(dot(C.cn, u0)) + (lo[4] + kBoxTol) * fabsf(dot(C.cn, u1)) +
+                         (lo[5] + kBoxTol) * fabsf(dot(C.cn, u2));
+        if (fabsf(dot(C.cn, oc) - C.cw) > rr) return false;
+        C.blo[0] = fminf(C.c0.x, fminf(C.c1.x, C.c2.x)) - kBoxTol; C.bhi[0] = fmaxf(C.c0.x, fmaxf(C.c1.x, C.c2.x)) + kBoxTol;
+        C.blo[1] = fminf(C.c0.y, fminf(C.c1.y, C.c2.y)) - kBoxTol; C.bhi[1] = fmaxf(C.c0.y, fmaxf(C.c1.y, C.c2.y)) + kBoxTol;
+        C.blo[2] = fminf(C.c0.z, fminf(C.c1.z, C.c2.z)) - kBoxTol; C.bhi[2] = fmaxf(C.c0.z, fmaxf(C.c1.z, C.c2.z)) + kBoxTol;
+        C.big = fmaxf(fmaxf(C.bhi[0] - C.blo[0], C.bhi[1] - C.blo[1]), C.bhi[2] - C.blo[2]) > kBigTri;
+        return true;
+    }
+    const float4* e = wp + 2ull * prim;
+    C.c0 = xf_inv(C.T, f3of(__ldg(e)));
+    C.c1 = xf_inv(C.T, f3of(__ldg(e + 1)));
+    const f3 d = C.c1 - C.c0;
+    C.cinv = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+    const f3 pr = C.c0 - oc;
+    const f3 po = mk(dot(pr, u0), dot(pr, u1), dot(pr, u2));
+    const f3 dd = mk(dot(d, u0), dot(d, u1), dot(d, u2));
+    Box obl;
+    obl.lo[0] = -lo[3]; obl.lo[1] = -lo[4]; obl.lo[2] = -lo[5];
+    obl.hi[0] = lo[3]; obl.hi[1] = lo[4]; obl.hi[2] = lo[5];
+    return seg_box(po, mk(safe_inv(dd.x), safe_inv(dd.y), safe_inv(dd.z)), obl, kBoxTol);
+}
+
 // 0: nothing to do (blank, decided, overflowed item, empty link, OBB reject); 1: descend.
 // Every outcome but "decided" is a function of the inputs alone, so a warp
 // that sets up one candidate on all lanes (check_decided false) agrees.
@@ -644,7 +689,6 @@ template <bool R2O>
 __device__ __forceinline__ int stage_b_setup(const RobotDev& R, const SceneDev& S, const WaveArgs& W, uint2 cd,
                                              StageBCand& C, unsigned long long& n_skip, unsigned long long& n_rej,
                                              bool check_decided = true) {
-    constexpr float kBoxTol = 2e-5f;
     const DiscreteArgs& A = W.d;
     if (cd.x == kNone) return 0;  // blank slot of an overflowed emission
     const uint32_t item = cd.x;
@@ -657,49 +701,11 @@ __device__ __forceinline__ int stage_b_setup(const RobotDev& R, const SceneDev& 
     C.lroot = R2O ? R.edge_root[link] : R.tri_root[link];
     if (C.lroot == kNone) return 0;
     C.pose = pose;
-    C.prim = cd.y;
     const float4* tp = A.T + ((size_t) pose * R.n_links + link) * 3;
     C.T[0] = tp[0]; C.T[1] = tp[1]; C.T[2] = tp[2];
-    const float* lo = R.obb[link];
-    const f3 oc = mk(lo[0], lo[1], lo[2]);
-    const f3 u0 = mk(lo[6], lo[7], lo[8]), u1 = mk(lo[9], lo[10], lo[11]), u2 = mk(lo[12], lo[13], lo[14]);
-    const float4* __restrict__ wp = R2O ? S.tri_prims : S.edge_prims;
-    C.c2 = C.cn = C.cinv = mk(0.f, 0.f, 0.f);
-    C.cw = 0.f;
-    C.big = false;
-    if (R2O) {
-        const float4* t = wp + 3ull * cd.y;
-        C.c0 = xf_inv(C.T, f3of(__ldg(t)));
-        C.c1 = xf_inv(C.T, f3of(__ldg(t + 1)));
-        C.c2 = xf_inv(C.T, f3of(__ldg(t + 2)));
-        C.cn = cross(C.c1 - C.c0, C.c2 - C.c0);
-        C.cw = dot(C.cn, C.c0);
-        const float rr = (lo[3] + kBoxTol) * fabsf(dot(C.cn, u0)) + (lo[4] + kBoxTol) * fabsf(dot(C.cn, u1)) +
-                         (lo[5] + kBoxTol) * fabsf(dot(C.cn, u2));
-        if (fabsf(dot(C.cn, oc) - C.cw) > rr) {
-            ++n_rej;
-            return 0;
-        }
-        C.blo[0] = fminf(C.c0.x, fminf(C.c1.x, C.c2.x)) - kBoxTol; C.bhi[0] = fmaxf(C.c0.x, fmaxf(C.c1.x, C.c2.x)) + kBoxTol;
-        C.blo[1] = fminf(C.c0.y, fminf(C.c1.y, C.c2.y)) - kBoxTol; C.bhi[1] = fmaxf(C.c0.y, fmaxf(C.c1.y, C.c2.y)) + kBoxTol;
-        C.blo[2] = fminf(C.c0.z, fminf(C.c1.z, C.c2.z)) - kBoxTol; C.bhi[2] = fmaxf(C.c0.z, fmaxf(C.c1.z, C.c2.z)) + kBoxTol;
-        C.big = fmaxf(fmaxf(C.bhi[0] - C.blo[0], C.bhi[1] - C.blo[1]), C.bhi[2] - C.blo[2]) > kBigTri;
-    } else {
-        const float4* e = wp + 2ull * cd.y;
-        C.c0 = xf_inv(C.T, f3of(__ldg(e)));
-        C.c1 = xf_inv(C.T, f3of(__ldg(e + 1)));
-        const f3 d = C.c1 - C.c0;
-        C.cinv = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-        const f3 pr = C.c0 - oc;
-        const f3 po = mk(dot(pr, u0), dot(pr, u1), dot(pr, u2));
-        const f3 dd = mk(dot(d, u0), dot(d, u1), dot(d, u2));
-        Box obl;
-        obl.lo[0] = -lo[3]; obl.lo[1] = -lo[4]; obl.lo[2] = -lo[5];
-        obl.hi[0] = lo[3]; obl.hi[1] = lo[4]; obl.hi[2] = lo[5];
-        if (!seg_box(po, mk(safe_inv(dd.x), safe_inv(dd.y), safe_inv(dd.z)), obl, kBoxTol)) {
-            ++n_rej;
-            return 0;
-        }
+    if (!cand_geometry<R2O>(R, S, link, cd.y, C)) {
+        ++n_rej;
+        return 0;
     }
     return 1;
 }
@@ -969,25 +975,6 @@ __global__ void __launch_bounds__(BLOCK) k_stage_b_packet(const RobotDev R, cons
     warp_count(A.stats + 7, n_node);
 }
 
-// Stages A and B in one warp per (pose, link) item.  The warp descends the
-// scene's 4-wide tree with the link's OBB through a shared LIFO frontier
-// (each step pops up to 32 nodes and spreads their children over the lanes:
-// 4 lanes per node when at most 8 are waiting, 2 when at most 16, else one
-// lane tests all four children of its node, so a step costs about one box
-// test per lane and the descent half the dependent node loads of a binary
-// tree), keeps the leaf survivors in a shared buffer and, 32 at a time, runs
-// them through stage B at once (one lane per candidate, bounded by the light
-// budget; longer candidates are written to the candidate buffer and handed
-// to the heavy pass).  An item whose pose is found in collision stops
-// generating candidates: most colliding items are decided after their first
-// few candidates, so most of stage A's traversal and candidate traffic is
-// never spent on them.  PACKET: the 32 buffered candidates (one item, so one
-// link tree) descend the link LBVH together - one node load per step for the
-// warp, each lane testing its own primitive - which shares the top levels of
-// the link tree when many small scene primitives crowd one link.
-constexpr int kAbWarps = 4;
-constexpr int kCandBuf = 32 + 32 * kWide;  // < 32 waiting + up to 32 * kWide added by one frontier step
-
 // The link OBB of an item in the world frame, padded by the box tolerance,
 // and its world-axis half extents.
 __device__ __forceinline__ void item_box(const RobotDev& R, const DiscreteArgs& A, uint32_t pose, uint32_t link,
@@ -1003,363 +990,491 @@ __device__ __forceinline__ void item_box(const RobotDev& R, const DiscreteArgs& 
              fabsf(ob.ax[0].z) * ob.h.x + fabsf(ob.ax[1].z) * ob.h.y + fabsf(ob.ax[2].z) * ob.h.z);
 }
 
-// Marks an item for the thread-per-item fallback once, however many warps
-// give up on it (one byte per item in a word-aligned buffer with 3 spare bytes).
-__device__ __forceinline__ void mark_overflow(const WaveArgs& W, uint32_t item) {
-    unsigned* word = reinterpret_cast<unsigned*>(W.item_overflow + (item & ~3u));
-    const unsigned bit = 1u << (8 * (item & 3u));
-    if (!(atomicOr(word, bit) & bit)) W.overflow_items[atomicAdd(W.overflow_count, 1u)] = item;
+template <class K>
+static uint32_t grid_for(K kernel, int threads) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
+    return (uint32_t) std::max(1, per_sm) * (uint32_t) device_sm_count();
 }
 
-// The OBB test of the wide descents (wide.cuh) of the fused and subtree kernels.
+// ---------------------------------------------------------------- the query kernel
+// Both stages in one persistent launch, one warp per task.  A task is a (pose,
+// link) item from the culled list, or a part of one: a scene-tree node that a
+// busy warp handed to an idle one.
+//
+// Stage A: the warp descends the scene's 4-wide tree with the link's world OBB
+// through a frontier in shared memory (wide.cuh) and collects the overlapping
+// scene primitives.  Stage B takes them 32 at a time: each is moved into the
+// link frame and its geometry kept in shared memory, one column per candidate;
+// then the warp descends the link's 4-wide tree with all of them at once, its
+// frontier holding (candidate, node) pairs, and tests the (candidate, link
+// primitive) pairs it reaches 32 at a time.  Lanes take pairs, not candidates,
+// so they stay busy while any pair waits, whichever candidate it belongs to,
+// and no lane keeps a stack.  (One lane per candidate with a stack in local
+// memory left 15 of 32 lanes active and handed long descents to passes of
+// their own.)
+//
+// Load balance: a warp that finds the item list empty takes a ticket and waits
+// on that ticket's slot.  A busy warp that sees more tickets taken than tasks
+// offered hands the oldest nodes of its scene frontier, its largest subtrees,
+// to the waiting warps, one each; so the work of one crowded item spreads over
+// the GPU while the others finish, in flag and in count mode alike.  (Pairs and
+// candidates are not handed on: such tasks cost more than they take.)  The warp
+// whose ticket makes every live warp a waiting one ends all of them.  Live are
+// the warps of the blocks that have started: blocks still waiting for room
+// beside another launch's are not waited for, and find the list empty when they
+// come.  A waiting warp gives up after a bounded time; what is offered to a
+// ticket that was given up stays with the warp that offered it, so no task
+// depends on a waiter.
+constexpr int kFrontCap = 512;   // scene nodes waiting (frontier_reserve(kMaxTreeDepth) = 190)
+constexpr int kPairCap = 512;    // (candidate, link node) pairs waiting
+constexpr int kCandBuf = 32 + 32 * kWide;  // < 32 waiting + up to 32 * kWide added by one frontier step
+constexpr int kQueryPolls = 1 << 16;       // polls of a slot (at least 200 ns apart) before a waiting warp gives up
+
+// A slot is two 64-bit words, each with the ticket (plus one) it was written
+// for in its high half, so a reader knows from each word alone whether it is
+// the one it waits for and no fence orders them.  Second word: the scene node.
+// First word: the item, or what became of the ticket.
+constexpr uint32_t kTaken = 0xFFFFFFFFu, kGivenUp = 0xFFFFFFFEu, kOver = 0xFFFFFFFDu;
+__device__ __forceinline__ unsigned long long slot_word(uint32_t t, uint32_t v) {
+    return ((unsigned long long) (t + 1) << 32) | v;
+}
+__device__ __forceinline__ unsigned long long slot_empty(uint32_t t, uint32_t slots) {
+    return t < slots ? 0ull : slot_word(t - slots, kTaken);
+}
+
+// Tickets taken beyond the tasks offered: warps waiting for work.
+__device__ __forceinline__ int waiting(unsigned long long q) { return (int) ((uint32_t) q - (uint32_t) (q >> 32)); }
+
+// Ends the launch when every live warp waits (all lanes call): the tickets taken
+// so far count as served, and their slots are marked.
+__device__ __forceinline__ void end_if_all_wait(const QueryArgs& Q) {
+    const int lane = threadIdx.x & 31;
+    int ended = 0;
+    uint32_t first = 0;
+    if (lane == 0) {
+        __threadfence();  // this warp's ticket, or its leaving, before what it sees of the others
+        for (int tries = 0; tries < 64; ++tries) {
+            const unsigned long long q = *(volatile unsigned long long*) Q.queue;
+            const int waits = waiting(q);
+            if (waits <= 0 || waits < (int) *(volatile uint32_t*) Q.live) break;
+            if (atomicCAS(Q.queue, q, q + ((unsigned long long) waits << 32)) == q) {
+                atomicSub(Q.live, (uint32_t) waits);
+                ended = waits;
+                first = (uint32_t) (q >> 32);
+                break;
+            }
+        }
+    }
+    ended = __shfl_sync(0xffffffffu, ended, 0);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    for (int k = lane; k < ended; k += 32) {
+        const uint32_t i = first + k;
+        atomicCAS(&Q.slot[i & (Q.slots - 1)].x, slot_empty(i, Q.slots), slot_word(i, kOver));
+    }
+    __syncwarp();
+}
+
+// A task for an idle warp (all lanes call): (item, scene node); false when it is
+// to leave: the launch is over, or enough warps wait already (Q.most_waiting).
+__device__ __forceinline__ bool take_task(const QueryArgs& Q, uint2& task) {
+    const int lane = threadIdx.x & 31;
+    uint32_t t = 0, leave = 0;
+    if (lane == 0) {
+        leave = waiting(*(volatile unsigned long long*) Q.queue) >= (int) Q.most_waiting;
+        if (leave) atomicSub(Q.live, 1u);
+        else t = (uint32_t) atomicAdd(Q.queue, 1ull);
+    }
+    leave = __shfl_sync(0xffffffffu, leave, 0);
+    end_if_all_wait(Q);
+    if (leave) return false;
+    uint32_t got = 0;
+    if (lane == 0) {
+        ulonglong2* slot = Q.slot + (t & (Q.slots - 1));
+        uint32_t nap = 100;
+        int polls = 0;
+        unsigned long long w;
+        while (true) {
+            w = *(volatile unsigned long long*) &slot->x;
+            if ((uint32_t) (w >> 32) == t + 1) break;
+            if (++polls > kQueryPolls) {  // gives up, unless a task arrives just now
+                w = atomicCAS(&slot->x, slot_empty(t, Q.slots), slot_word(t, kGivenUp));
+                if ((uint32_t) (w >> 32) != t + 1) atomicSub(Q.live, 1u);
+                break;
+            }
+            __nanosleep(nap);
+            nap = min(2 * nap, 800u);
+        }
+        if ((uint32_t) (w >> 32) == t + 1 && (uint32_t) w < kOver) {
+            task.x = (uint32_t) w;
+            // written before the first word, so it is here or on its way
+            for (polls = 0; polls < kQueryPolls; ++polls) {
+                w = *(volatile unsigned long long*) &slot->y;
+                if ((uint32_t) (w >> 32) == t + 1) break;
+            }
+            task.y = (uint32_t) w;
+            got = 1;
+            atomicExch(&slot->x, slot_word(t, kTaken));
+        }
+    }
+    task.x = __shfl_sync(0xffffffffu, task.x, 0);
+    task.y = __shfl_sync(0xffffffffu, task.y, 0);
+    return __shfl_sync(0xffffffffu, got, 0) != 0;
+}
+
+// Hands up to `want` (at most 32) of the oldest of the scene nodes fr[0, sp) to
+// waiting warps.
+__device__ __forceinline__ void offer_tasks(const QueryArgs& Q, int want, uint32_t item, uint32_t* fr, int& sp) {
+    const int lane = threadIdx.x & 31;
+    const int give = min(want, 32);
+    uint32_t t0 = 0;
+    if (lane == 0) t0 = (uint32_t) (atomicAdd(Q.queue, (unsigned long long) give << 32) >> 32);
+    t0 = __shfl_sync(0xffffffffu, t0, 0);
+    uint32_t node = 0;
+    bool kept = false;
+    if (lane < give) {
+        node = fr[lane];
+        const uint32_t t = t0 + lane;
+        ulonglong2* slot = Q.slot + (t & (Q.slots - 1));
+        const unsigned long long empty = slot_empty(t, Q.slots);
+        // a slot's last user may be about to mark it taken (it has its task): a short, bounded wait
+        for (int polls = 0; polls < 4096; ++polls) {
+            const unsigned long long w = *(volatile unsigned long long*) &slot->x;
+            if (w == empty || w == slot_word(t, kGivenUp)) break;
+        }
+        *(volatile unsigned long long*) &slot->y = slot_word(t, node);
+        kept = atomicCAS(&slot->x, empty, slot_word(t, item)) != empty;
+    }
+    const uint32_t mk_ = __ballot_sync(0xffffffffu, kept);
+    const int back = __popc(mk_);
+    // the nodes kept, then the rest moved down
+    for (int i = 0; i < sp - give; i += 32) {
+        const bool on = i + lane < sp - give;
+        const uint32_t v = on ? fr[give + i + lane] : 0u;
+        __syncwarp();
+        if (on) fr[back + i + lane] = v;
+        __syncwarp();
+    }
+    if (kept) fr[__popc(mk_ & ((1u << lane) - 1u))] = node;
+    sp -= give - back;
+    __syncwarp();
+}
+
+// The OBB test of the scene descents; the warp's box lives in shared memory
+// and is read at every step, so that no register holds it during stage B.
+struct ObbCol {
+    float4 v[5];  // centre, half sizes, axes x y z, world half extents: 18 values
+    __device__ __forceinline__ void put(const ObbW& o, const f3& e) {
+        v[0] = make_float4(o.c.x, o.c.y, o.c.z, o.h.x);
+        v[1] = make_float4(o.h.y, o.h.z, o.ax[0].x, o.ax[0].y);
+        v[2] = make_float4(o.ax[0].z, o.ax[1].x, o.ax[1].y, o.ax[1].z);
+        v[3] = make_float4(o.ax[2].x, o.ax[2].y, o.ax[2].z, e.x);
+        v[4] = make_float4(e.y, e.z, 0.f, 0.f);
+    }
+};
 struct ObbTest {
-    const ObbW& ob;
-    const f3& ext;
+    const ObbCol& col;
+    ObbW ob;
+    f3 ext;
+    __device__ __forceinline__ explicit ObbTest(const ObbCol& c) : col(c) {}
+    __device__ __forceinline__ void bind(uint32_t) {
+        const float4 a = col.v[0], b = col.v[1], c = col.v[2], d = col.v[3], e = col.v[4];
+        ob.c = mk(a.x, a.y, a.z);
+        ob.h = mk(a.w, b.x, b.y);
+        ob.ax[0] = mk(b.z, b.w, c.x);
+        ob.ax[1] = mk(c.y, c.z, c.w);
+        ob.ax[2] = mk(d.x, d.y, d.z);
+        ext = mk(d.w, e.x, e.y);
+    }
     __device__ __forceinline__ bool operator()(const Box& b) const { return obb_aabb(b, ob, ext); }
 };
 
-// Register caps (measured on the 65,536-pose dense workload and the dense
-// shelf): RobotToObs at 5 resident blocks per SM (96 registers, a few spills;
-// more warps to hide the node-load latency: 4 blocks at 128 registers was 7 %
-// slower), ObsToRobot at 4 (128 registers, no spills: 2-4 % faster than 5).
-// TOP: the first W.top_nodes wide nodes are staged in shared memory after the
-// frontiers and read from there (a separate instantiation, so the default
-// kernel's node loads carry no branch).
-template <bool R2O, bool PACKET, bool TOP>
-__global__ void __launch_bounds__(kAbWarps * 32, R2O ? 5 : 4) k_stage_ab(const RobotDev R, const SceneDev S, const WaveArgs W) {
-    extern __shared__ uint32_t s_front[];  // [kAbWarps][S.wide_front], then (TOP) the staged wide nodes
-    __shared__ uint32_t s_cand[kAbWarps][kCandBuf];
-    __shared__ uint32_t s_hits[kAbWarps];  // a lane of the warp's current stage-B step hit its pose
-    const DiscreteArgs& A = W.d;
+// The candidates of a stage-B batch in shared memory: [field][candidate].
+template <bool R2O>
+struct CandCols {
+    static constexpr int kFields = R2O ? 20 : 10;  // the last: the scene primitive
+    float f[kFields][32];
+    __device__ __forceinline__ void put(int c, const StageBCand& C) {
+        f[0][c] = C.c0.x; f[1][c] = C.c0.y; f[2][c] = C.c0.z;
+        f[3][c] = C.c1.x; f[4][c] = C.c1.y; f[5][c] = C.c1.z;
+        if (R2O) {
+            f[6][c] = C.c2.x; f[7][c] = C.c2.y; f[8][c] = C.c2.z;
+            f[9][c] = C.cn.x; f[10][c] = C.cn.y; f[11][c] = C.cn.z;
+            f[12][c] = C.cw;
+            for (int k = 0; k < 3; ++k) {
+                f[13 + k][c] = C.blo[k];
+                f[16 + k][c] = C.bhi[k];
+            }
+        } else {
+            f[6][c] = C.cinv.x; f[7][c] = C.cinv.y; f[8][c] = C.cinv.z;
+        }
+        f[kFields - 1][c] = __uint_as_float(C.prim);
+    }
+    __device__ __forceinline__ f3 vec(int k, uint32_t c) const { return mk(f[k][c], f[k + 1][c], f[k + 2][c]); }
+};
+
+template <bool R2O>
+struct PairTest {
+    const CandCols<R2O>& cols;
+    StageBCand C;
+    uint32_t col;
+    __device__ __forceinline__ explicit PairTest(const CandCols<R2O>& k) : cols(k) {}
+    __device__ __forceinline__ void bind(uint32_t c) {
+        col = c;
+        if (R2O) {
+            C.cn = cols.vec(9, c);
+            C.cw = cols.f[12][c];
+            for (int k = 0; k < 3; ++k) {
+                C.blo[k] = cols.f[13 + k][c];
+                C.bhi[k] = cols.f[16 + k][c];
+            }
+            C.big = fmaxf(fmaxf(C.bhi[0] - C.blo[0], C.bhi[1] - C.blo[1]), C.bhi[2] - C.blo[2]) > kBigTri;
+        } else {
+            C.c0 = cols.vec(0, c);
+            C.cinv = cols.vec(6, c);
+        }
+    }
+    __device__ __forceinline__ bool operator()(const Box& b) const {
+        if (!stage_b_node<R2O, false>(C, b)) return false;
+        // a large triangle's corners are read only where its edges matter
+        return !R2O || !C.big || tri_box_edges(cols.vec(0, col), cols.vec(3, col), cols.vec(6, col), b, 2e-5f);
+    }
+};
+
+template <bool R2O>
+struct QueryWarp {
+    ObbCol obb;
+    uint32_t front[kFrontCap];
+    uint32_t pairs[kPairCap];
+    uint32_t cand[kCandBuf];
+    uint32_t leaf[kCandBuf];
+    CandCols<R2O> cols;
+};
+
+template <bool R2O, int PER_SM>
+__global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotDev R, const SceneDev S, const QueryArgs Q) {
+    __shared__ QueryWarp<R2O> s_warp[kQueryWarps];
+    __shared__ volatile uint32_t s_live;
+    const DiscreteArgs& A = Q.d;
     const int lane = threadIdx.x & 31;
-    uint32_t* fr = s_front + (threadIdx.x >> 5) * S.wide_front;
-    uint32_t* cb = s_cand[threadIdx.x >> 5];
-    volatile uint32_t* s_hit = s_hits + (threadIdx.x >> 5);
     const uint32_t lt = (1u << lane) - 1u;
+    QueryWarp<R2O>& s = s_warp[threadIdx.x >> 5];
     const float4* __restrict__ wn = R2O ? S.tri_wide : S.edge_wide;
     const float4* __restrict__ wp = R2O ? S.tri_prims : S.edge_prims;
     const uint32_t wroot = R2O ? S.tri_wide_root : S.edge_wide_root;
-    const float4* __restrict__ ln = R2O ? R.edge_nodes : R.tri_nodes;
+    const float4* __restrict__ ln = R2O ? R.edge_wide : R.tri_wide;
     const float4* __restrict__ lp = R2O ? R.edge_prims : R.tri_prims;
-    const uint32_t n_items = *A.n_items;
-    const uint32_t budget = W.light_steps ? W.light_steps : 0xFFFFFFFFu;
-    // the tree's top levels in shared memory (its first nodes, breadth-first), read by every descent
-    const uint32_t n_top = TOP ? min(W.top_nodes, R2O ? S.n_tri_wide : S.n_edge_wide) : 0u;
-    float4* s_top = reinterpret_cast<float4*>(s_front + ((kAbWarps * S.wide_front + 3u) & ~3u));
-    if constexpr (TOP) {
-        for (uint32_t k = threadIdx.x; k < n_top * 2 * kWide; k += blockDim.x) s_top[k] = __ldg(wn + k);
-        __syncthreads();
-    }
-    uint32_t st[kStack];
-    unsigned long long n_acc = 0, n_skip = 0, n_rej = 0, n_leaf = 0, n_cand = 0, n_node = 0;
+    const int reserve_a = (int) frontier_reserve(R2O ? S.tri_wide_depth : S.edge_wide_depth);
+    const int reserve_b = (int) frontier_reserve(R2O ? R.edge_wide_depth : R.tri_wide_depth);
+    const uint32_t n_items = *A.n_items, warps = gridDim.x * kQueryWarps;
+    const bool counting = A.want_counts != 0;
+    if (threadIdx.x == 0) s_live = 0;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(Q.live, (uint32_t) kQueryWarps) != kNone) s_live = 1;  // set once it has returned
+    uint32_t n_leaf = 0, n_cand = 0, n_node = 0;
+    bool listed = wroot != kNone;  // the item list may hold more
+    uint32_t first = blockIdx.x * kQueryWarps + (threadIdx.x >> 5);  // the warp's first item; kNone: taken
     while (true) {
-        uint32_t it = 0;
-        if (lane == 0) it = atomicAdd(A.work_counter, 1u);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= n_items) break;
-        const uint32_t item = item_word(A, R.n_links, A.items[it]);
-        const uint32_t pose = item / R.n_links, link = item - pose * R.n_links;
+        uint2 task = make_uint2(0u, kNone);  // (item word, scene node; kNone: the whole item)
+        uint32_t poll = 1;                   // steps between looks at the queue
+        if (listed) {
+            uint32_t it = first;
+            if (it == kNone) {
+                if (lane == 0) it = warps + atomicAdd(A.work_counter, 1u);
+                it = __shfl_sync(0xffffffffu, it, 0);
+            }
+            first = kNone;
+            if (it < n_items) {
+                task.x = item_word(A, R.n_links, A.items[it]);
+                if (n_items - it > warps) poll = 4;
+            } else {
+                listed = false;
+                for (int polls = 0; !s_live && polls < kQueryPolls; ++polls) {}  // live before idle
+            }
+        }
+        if (!listed && !take_task(Q, task)) break;
+        const uint32_t item = task.x, pose = item / R.n_links, link = item - pose * R.n_links;
         if (pose >= A.n_poses) {
             if (lane == 0) atomicOr(A.err, kErrRange);
             continue;
         }
-        uint32_t dec = 0;
-        if (lane == 0 && !A.want_counts) dec = ld_flag(A.pose_hit + pose);
-        if (wroot == kNone || __shfl_sync(0xffffffffu, dec, 0)) continue;
-        ObbW ob;
-        f3 ext;
-        item_box(R, A, pose, link, ob, ext);
-        // the descent starts with the tree's top cut; a one-primitive scene's root is its only candidate
+        uint32_t decided = 0;
+        if (lane == 0 && !counting) decided = ld_flag(A.pose_hit + pose);
+        unsigned long long queue = 0;
+        if (lane == 0) queue = *(volatile unsigned long long*) Q.queue;
+        const uint32_t lroot = R2O ? R.edge_wide_root[link] : R.tri_wide_root[link];
+        {
+            ObbW ob;
+            f3 ext;
+            item_box(R, A, pose, link, ob, ext);
+            if (__shfl_sync(0xffffffffu, decided, 0) || lroot == kNone) continue;
+            if (lane == 0) s.obb.put(ob, ext);
+            __syncwarp();
+        }
+        ObbTest obb_test(s.obb);
         int sp = 0, nc = 0;
-        uint32_t nbs = 0;  // stage-B steps this item ran in its warp
-        bool overflow = false;
-        if (wroot & kLeaf) {
-            if (lane == 0) cb[0] = wroot & ~kLeaf;
+        uint32_t hits = 0, tick = 0;
+        if (task.y != kNone) {
+            if (lane == 0) s.front[0] = task.y;
+            sp = 1;
+            __syncwarp();
+        } else if (wroot & kLeaf) {
+            if (lane == 0) s.cand[0] = wroot & ~kLeaf;
             nc = 1;
             __syncwarp();
-        } else if (!cut_step(R2O ? S.tri_cut : S.edge_cut, R2O ? S.n_tri_cut : S.n_edge_cut, fr, sp, cb, nc,
-                             ObbTest{ob, ext}, S.wide_front, A.err, n_node, n_cand)) {
+        } else if (!frontier_cut(R2O ? S.tri_cut : S.edge_cut, R2O ? S.n_tri_cut : S.n_edge_cut, s.front, sp, s.cand, nc,
+                                 obb_test, kFrontCap, A.err, n_node)) {
             continue;
         }
+        if (lane == 0) n_cand += nc;
+        auto share = [&](int most) {  // hands up to `most` nodes of the scene frontier to waiting warps
+            const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
+            if (want > 0 && most > 0) offer_tasks(Q, min(want, most), item, s.front, sp);
+            if (lane == 0) queue = *(volatile unsigned long long*) Q.queue;
+        };
         while (true) {
-            if (nc >= 32 || (sp == 0 && nc > 0)) {  // stage B on up to 32 buffered candidates
-                const int take = min(nc, 32);
-                nc -= take;
-                const uint32_t prim = lane < take ? cb[nc + lane] : kNone;
-                __syncwarp();
-                if (!A.want_counts && nbs >= W.item_steps) {
-                    // a crowded item: its further candidates go to the one-lane pass, which
-                    // spreads them over the whole GPU instead of this warp's serial steps
-                    uint32_t base = 0, d2 = 0;
-                    if (lane == 0) {
-                        d2 = ld_flag(A.pose_hit + pose);  // decided by another item: stop enumerating
-                        if (!d2) base = atomicAdd(W.cand_count, (uint32_t) take);
-                    }
-                    if (__shfl_sync(0xffffffffu, d2, 0)) break;
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    if (base + (uint32_t) take <= W.cand_cap) {
-                        if (prim != kNone) W.cand[base + lane] = make_uint2(item, prim);
-                        if (sp > 0) {
-                            // and the rest of its descent to the subtree pass, one warp per frontier
-                            // node, so no single warp walks a crowded item's whole overlap
-                            uint32_t sb = 0;
-                            if (lane == 0) sb = atomicAdd(W.sub_count, (uint32_t) sp);
-                            sb = __shfl_sync(0xffffffffu, sb, 0);
-                            const bool fits = sb + (uint32_t) sp <= W.sub_cap;
-                            for (int i = lane; i < sp; i += 32)  // slots below the capacity are always written
-                                if (sb + i < W.sub_cap) W.sub[sb + i] = fits ? make_uint2(item, fr[i]) : make_uint2(kNone, kNone);
-                            __syncwarp();
-                            if (!fits) {
-                                overflow = true;
-                                break;
-                            }
-                            sp = 0;
-                        }
-                        continue;
-                    }
-                    // no room: blank the reserved slots below the capacity and hand the whole
-                    // item to the thread-per-item kernel (flags only, so re-running is safe)
-                    if (prim != kNone && base + lane < W.cand_cap) W.cand[base + lane] = make_uint2(kNone, kNone);
-                    overflow = true;
-                    break;
+            if (nc < 32 && sp > 0) {  // stage A
+                if (++tick >= poll) {
+                    tick = 0;
+                    share(sp - 1);
                 }
-                ++nbs;
-                bool hit = false;
-                StageBCand C;
-                if (lane == 0) *s_hit = 0u;
-                __syncwarp();
-                if (PACKET) {
-                    const bool live =
-                        prim != kNone && stage_b_setup<R2O>(R, S, W, make_uint2(item, prim), C, n_skip, n_rej, false);
-                    const uint32_t grp = __ballot_sync(0xffffffffu, live);
-                    if (live) ++n_acc;
-                    if (grp) {
-                        int bsp = 0;
-                        st[bsp++] = R2O ? R.edge_root[link] : R.tri_root[link];
-                        uint32_t steps = 0, hits = 0;
-                        bool spilled = false;
-                        const uint32_t rank = __popc(grp & lt), np = __popc(grp);
-                        while (bsp > 0) {
-                            if (++steps > 4u * budget) {  // hand the packet's candidates to the heavy pass
-                                uint32_t hbase = 0;
-                                if (lane == 0) hbase = atomicAdd(W.heavy_count, np);
-                                hbase = __shfl_sync(0xffffffffu, hbase, 0);
-                                const bool fits = hbase + np <= W.heavy_cap;
-                                // heavy slots below the capacity are always written (blank when the
-                                // packet stays here), since the heavy pass reads up to it
-                                if (live && hbase + rank < W.heavy_cap)
-                                    W.heavy[hbase + rank] = fits ? make_uint2(item, prim) : make_uint2(kNone, kNone);
-                                if (fits) {
-                                    spilled = true;
-                                    break;
-                                }
-                                steps = 0;  // no room: finish the packet here
-                            }
-                            const uint32_t ref = st[--bsp];
-                            if (ref & kLeaf) {
-                                const uint32_t li = ref & ~kLeaf;
-                                bool h = false;
-                                if (live) {
-                                    ++n_leaf;
-                                    h = stage_b_leaf<R2O>(lp, wp, li, C, A.stats);
-                                }
-                                if (__any_sync(0xffffffffu, h)) {
-                                    hit = true;
-                                    if (!A.want_counts) break;
-                                    if (h) {
-                                        if (R2O) {
-                                            const uint32_t eid = __float_as_uint(__ldg(lp + 2ull * li).w);
-                                            atomicOr(A.edge_bits + (size_t) pose * A.edge_words + (eid >> 5),
-                                                     1u << (eid & 31));
-                                        } else {
-                                            ++hits;
-                                        }
-                                    }
-                                }
-                                continue;
-                            }
-                            Box bl, br;
-                            uint32_t rl, rr;
-                            load_node(ln, ref, bl, br, rl, rr);
-                            if (live) n_node += 2;
-                            const bool hr = live && stage_b_node<R2O>(C, br), hl = live && stage_b_node<R2O>(C, bl);
-                            const bool any_r = __any_sync(0xffffffffu, hr), any_l = __any_sync(0xffffffffu, hl);
-                            if (bsp + 2 > kStack) {
-                                if (lane == 0) atomicOr(A.err, kErrStack);
-                                break;
-                            }
-                            if (any_r) st[bsp++] = rr;
-                            if (any_l) st[bsp++] = rl;
-                        }
-                        if (hits && !spilled) atomicAdd(A.counts + pose, hits);
-                    }
-                } else if (prim != kNone && stage_b_setup<R2O>(R, S, W, make_uint2(item, prim), C, n_skip, n_rej, false)) {
-                    ++n_acc;
-                    int bsp = 0;
-                    st[bsp++] = C.lroot;
-                    uint32_t steps = 0, hits = 0;
-                    bool spilled = false;
-                    while (bsp > 0) {
-                        // flags only: another lane of this step has hit the pose, so the rest is moot
-                        if (!A.want_counts && *s_hit) break;
-                        if (++steps > budget) {
-                            const uint32_t h = atomicAdd(W.heavy_count, 1u);
-                            if (h < W.heavy_cap) {
-                                W.heavy[h] = make_uint2(item, prim);
-                                spilled = true;
-                                break;
-                            }
-                            steps = 0;  // no room: finish the candidate here
-                        }
-                        const uint32_t ref = st[--bsp];
-                        if (ref & kLeaf) {
-                            ++n_leaf;
-                            const uint32_t li = ref & ~kLeaf;
-                            if (stage_b_leaf<R2O>(lp, wp, li, C, A.stats)) {
-                                hit = true;
-                                if (!A.want_counts) {
-                                    *s_hit = 1u;
-                                    break;
-                                }
-                                if (R2O) {
-                                    const uint32_t eid = __float_as_uint(__ldg(lp + 2ull * li).w);
-                                    atomicOr(A.edge_bits + (size_t) pose * A.edge_words + (eid >> 5), 1u << (eid & 31));
-                                } else {
-                                    ++hits;
-                                }
-                            }
-                            continue;
-                        }
-                        Box bl, br;
-                        uint32_t rl, rr;
-                        load_node(ln, ref, bl, br, rl, rr);
-                        n_node += 2;
-                        const bool hr = stage_b_node<R2O>(C, br), hl = stage_b_node<R2O>(C, bl);
-                        if (bsp + 2 > kStack) {
-                            atomicOr(A.err, kErrStack);
-                            break;
-                        }
-                        if (hr) st[bsp++] = rr;
-                        if (hl) st[bsp++] = rl;
-                    }
-                    if (hits && !spilled) atomicAdd(A.counts + pose, hits);
-                }
-                const bool any = __any_sync(0xffffffffu, hit);
-                if (any) {
-                    if (lane == 0) {
-                        if (A.want_counts) A.pose_hit[pose] = 1u;
-                        else atomicExch(A.pose_hit + pose, 1u);
-                    }
-                    if (!A.want_counts) break;
-                }
-                if (!A.want_counts) {  // decided meanwhile by another item?
-                    uint32_t d2 = 0;
-                    if (lane == 0) d2 = ld_flag(A.pose_hit + pose);
-                    if (__shfl_sync(0xffffffffu, d2, 0)) break;
-                }
+                const int nc0 = nc;
+                if (!frontier_step<false>(wn, s.front, sp, s.cand, nc, obb_test, kFrontCap, reserve_a, A.err, n_node)) break;
+                if (lane == 0) n_cand += nc - nc0;
                 continue;
             }
-            if (sp == 0) break;
-            if (!wide_step<TOP>(wn, fr, sp, cb, nc, ObbTest{ob, ext}, S.wide_front, A.err, n_node, n_cand, s_top, n_top))
-                break;
+            if (nc == 0) break;
+            // stage B on up to 32 candidates
+            if (lane == 0 && !counting) decided = ld_flag(A.pose_hit + pose);  // read now, looked at after the batch
+            const int take = min(nc, 32);
+            nc -= take;
+            int np = 0, nl = 0;
+            {
+                StageBCand C;
+                bool live = false;
+                if (lane < take) {
+                    const float4* tp = A.T + ((size_t) pose * R.n_links + link) * 3;
+                    C.T[0] = __ldg(tp); C.T[1] = __ldg(tp + 1); C.T[2] = __ldg(tp + 2);
+                    live = cand_geometry<R2O>(R, S, link, s.cand[nc + lane], C);
+                    if (live) s.cols.put(lane, C);
+                }
+                const uint32_t ml = __ballot_sync(0xffffffffu, live), tag = (uint32_t) lane << kTagShift;
+                if (lroot & kLeaf) {  // a one-primitive link
+                    if (live) s.leaf[__popc(ml & lt)] = tag | (lroot & ~kLeaf);
+                    nl = __popc(ml);
+                } else {
+                    if (live) s.pairs[__popc(ml & lt)] = tag | lroot;
+                    np = __popc(ml);
+                }
+                __syncwarp();
+            }
+            PairTest<R2O> pair_test(s.cols);
+            bool pose_hit = false;
+            while (true) {
+                if (nl < 32 && np > 0) {
+                    if (++tick >= poll) {
+                        tick = 0;
+                        share(sp);
+                    }
+                    if (!frontier_step<true>(ln, s.pairs, np, s.leaf, nl, pair_test, kPairCap, reserve_b, A.err, n_node)) break;
+                    continue;
+                }
+                if (nl == 0) break;
+                const int some = min(nl, 32);
+                nl -= some;
+                bool hit = false;
+                uint32_t li = 0;
+                if (lane < some) {
+                    const uint32_t e = s.leaf[nl + lane], c = e >> kTagShift;
+                    li = e & kTagRef;
+                    ++n_leaf;
+                    f3 p, q, a, b, t;
+                    if (R2O) {
+                        const float4* ed = lp + 2ull * li;
+                        p = f3of(__ldg(ed)); q = f3of(__ldg(ed + 1));
+                        a = s.cols.vec(0, c); b = s.cols.vec(3, c); t = s.cols.vec(6, c);
+                    } else {
+                        const float4* tr = lp + 3ull * li;
+                        p = s.cols.vec(0, c); q = s.cols.vec(3, c);
+                        a = f3of(__ldg(tr)); b = f3of(__ldg(tr + 1)); t = f3of(__ldg(tr + 2));
+                    }
+                    int r = seg_tri_f32(p, q, a, b, t);
+                    if (r == 2) {
+                        atomicAdd(A.stats, 1ull);
+                        r = retest_f64<R2O>(A.T + ((size_t) pose * R.n_links + link) * 3, lp, li, wp,
+                                            __float_as_uint(s.cols.f[CandCols<R2O>::kFields - 1][c]))
+                                ? 1 : 0;
+                    }
+                    hit = r == 1;
+                    if (R2O && hit && counting) {
+                        const uint32_t eid = __float_as_uint(__ldg(lp + 2ull * li).w);
+                        atomicOr(A.edge_bits + (size_t) pose * A.edge_words + (eid >> 5), 1u << (eid & 31));
+                    }
+                }
+                const uint32_t mh = __ballot_sync(0xffffffffu, hit);
+                if (mh) {
+                    pose_hit = true;
+                    hits += __popc(mh);
+                    if (!counting) break;
+                }
+                __syncwarp();
+            }
+            __syncwarp();
+            if (pose_hit && lane == 0) {
+                if (counting) A.pose_hit[pose] = 1u;
+                else atomicExch(A.pose_hit + pose, 1u);
+            }
+            // a hit, or another warp's meanwhile, decides the pose
+            if (!counting && (pose_hit || __shfl_sync(0xffffffffu, decided, 0))) break;
         }
-        if (overflow && lane == 0) mark_overflow(W, item);
+        if (!R2O && counting && lane == 0 && hits) atomicAdd(A.counts + pose, hits);
         __syncwarp();
     }
-    warp_count(A.stats + 1, n_acc);
-    warp_count(A.stats + 2, n_skip);
-    warp_count(A.stats + 3, n_rej);
     warp_count(A.stats + 4, n_leaf);
     warp_count(A.stats + 7, n_node);
     warp_count(A.stats + 6, n_cand);
 }
 
-// The subtree pass: the rest of a crowded item's scene descent, one warp
-// per frontier node the fused kernel handed over.  Every leaf that overlaps
-// the item's OBB is appended to the candidate buffer for the one-lane pass
-// (32 or more at a time); a subtree stops when its pose is decided.  When the
-// buffer is full the item goes to the thread-per-item fallback (flags only,
-// like every deferral).  It runs twice.  The first launch (SPLIT) takes the
-// fused kernel's nodes and descends breadth-first - while at most 32 nodes
-// wait, every step pops them all, so the frontier holds one level - and as
-// soon as a level is wider than 32 nodes hands those nodes to the second
-// launch, which descends each to the end: a large subtree becomes many
-// pieces of equal depth on as many warps instead of one warp's serial walk.
-template <bool R2O, bool SPLIT>
-__global__ void __launch_bounds__(kAbWarps * 32) k_subtree(const RobotDev R, const SceneDev S, const WaveArgs W) {
-    extern __shared__ uint32_t s_front[];  // [kAbWarps][S.wide_front]
-    __shared__ uint32_t s_cand[kAbWarps][kCandBuf];
-    const DiscreteArgs& A = W.d;
-    const int lane = threadIdx.x & 31;
-    uint32_t* fr = s_front + (threadIdx.x >> 5) * S.wide_front;
-    uint32_t* cb = s_cand[threadIdx.x >> 5];
-    const float4* __restrict__ wn = R2O ? S.tri_wide : S.edge_wide;
-    const uint2* src = SPLIT ? W.sub : W.sub + W.sub_cap;  // the second half holds the split pieces
-    const uint32_t n_sub = min(SPLIT ? W.sub_count[0] : W.sub_count[2], W.sub_cap);
-    uint32_t* work = SPLIT ? W.sub_count + 1 : W.sub_count + 3;
-    unsigned long long n_node = 0, n_cand = 0;
-    while (true) {
-        uint32_t h = 0;
-        if (lane == 0) h = atomicAdd(work, 1u);
-        h = __shfl_sync(0xffffffffu, h, 0);
-        if (h >= n_sub) break;
-        const uint2 pr = src[h];
-        if (pr.x == kNone) continue;  // a blanked slot of a reservation that did not fit
-        const uint32_t item = pr.x, pose = item / R.n_links, link = item - pose * R.n_links;
-        if (pose >= A.n_poses) {
-            if (lane == 0) atomicOr(A.err, kErrRange);
-            continue;
-        }
-        uint32_t skip = 0;
-        if (lane == 0) skip = W.item_overflow[item] | ld_flag(A.pose_hit + pose);
-        if (__shfl_sync(0xffffffffu, skip, 0)) continue;  // re-run whole by the fallback, or decided
-        ObbW ob;
-        f3 ext;
-        item_box(R, A, pose, link, ob, ext);
-        int sp = 1, nc = 0;
-        if (lane == 0) fr[0] = pr.y;
-        __syncwarp();
-        while (true) {
-            if (nc >= 32 || (sp == 0 && nc > 0)) {  // flush every buffered candidate
-                uint32_t base = 0, dec = 0;
-                if (lane == 0) {
-                    dec = ld_flag(A.pose_hit + pose);
-                    if (!dec) base = atomicAdd(W.cand_count, (uint32_t) nc);
-                }
-                if (__shfl_sync(0xffffffffu, dec, 0)) break;
-                base = __shfl_sync(0xffffffffu, base, 0);
-                const bool fits = base + (uint32_t) nc <= W.cand_cap;
-                for (int i = lane; i < nc; i += 32)  // slots below the capacity are always written
-                    if (base + i < W.cand_cap) W.cand[base + i] = fits ? make_uint2(item, cb[i]) : make_uint2(kNone, kNone);
-                __syncwarp();
-                nc = 0;
-                if (!fits) {
-                    if (lane == 0) mark_overflow(W, item);
-                    break;
-                }
-                continue;
-            }
-            if (sp == 0) break;
-            if (SPLIT && sp > 32) {  // one level wider than a step: hand its nodes to the second launch
-                uint32_t sb = 0;
-                if (lane == 0) sb = atomicAdd(W.sub_count + 2, (uint32_t) sp);
-                sb = __shfl_sync(0xffffffffu, sb, 0);
-                const bool fits = sb + (uint32_t) sp <= W.sub_cap;
-                uint2* dst = W.sub + W.sub_cap;
-                for (int i = lane; i < sp; i += 32)  // slots below the capacity are always written
-                    if (sb + i < W.sub_cap) dst[sb + i] = fits ? make_uint2(item, fr[i]) : make_uint2(kNone, kNone);
-                __syncwarp();
-                if (!fits && lane == 0) mark_overflow(W, item);
-                sp = 0;
-                if (!fits) break;
-                continue;  // flush what is buffered, then the item is done here
-            }
-            if (!wide_step(wn, fr, sp, cb, nc, ObbTest{ob, ext}, S.wide_front, A.err, n_node, n_cand)) break;
-        }
-        __syncwarp();
-    }
-    warp_count(A.stats + 7, n_node);
-    warp_count(A.stats + 6, n_cand);
+// Blocks and instantiation for a batch of `items` at most (the cull leaves a
+// quarter to a third of them).  Five resident blocks per SM (96 registers, some
+// spilled) are the faster for large batches, three (168, none spilled) below
+// kQueryFew items an SM, where the latency of a warp's steps counts; a batch
+// that would leave most warps without an item gets fewer blocks still, since
+// starting and ending an idle warp costs about 5 ns and waiting warps split the
+// running items too finely (1,024 poses, ObsToRobot, 5k triangles: 147 us on all
+// blocks, 98 on two per SM).  Counting has no early exit, so its items are
+// larger.  One waiting warp per SM takes what the others hand on; more only load
+// the queue's words (4,096 poses 180 us with one per SM, 202 with all) and keep
+// blocks from leaving the SMs to other launches.  Whole checks of uniform poses at three / five blocks per SM, in us,
+// RobotToObs on the 428k-triangle scene: 4,096 poses 200 / 216, 8,192 253 / 263,
+// 16,384 397 / 373, 32,768 691 / 621; on the 202k-triangle shelf: 4,096 168 / 180,
+// 16,384 271 / 300, 32,768 393 / 395.
+constexpr uint32_t kQueryFew = 768;
+template <bool R2O>
+static void query_dispatch(const RobotDev& R, const SceneDev& S, const QueryArgs& Q, uint64_t items, uint32_t share,
+                           uint32_t most, cudaStream_t s) {
+    const uint32_t sms = (uint32_t) device_sm_count();
+    const bool few = items <= (uint64_t) kQueryFew * sms;
+    static const uint32_t fit_few = grid_for(k_query<R2O, 3>, kQueryWarps * 32);
+    static const uint32_t fit_all = grid_for(k_query<R2O, 5>, kQueryWarps * 32);
+    const uint64_t useful = std::max<uint64_t>(2 * sms, items / (Q.d.want_counts ? 4 : 64));
+    uint32_t blocks = (uint32_t) std::min<uint64_t>(std::max(1u, (few ? fit_few : fit_all) * share / 100), useful);
+    blocks = std::min({blocks, std::max(1u, most), kQuerySlots / (2 * kQueryWarps)});
+    QueryArgs G = Q;
+    G.most_waiting = sms;
+    if (few)
+        k_query<R2O, 3><<<blocks, kQueryWarps * 32, 0, s>>>(R, S, G);
+    else
+        k_query<R2O, 5><<<blocks, kQueryWarps * 32, 0, s>>>(R, S, G);
+    cuda_check(cudaGetLastError(), "k_query");
+}
+
+void launch_query(bool r2o, const RobotDev& R, const SceneDev& S, const QueryArgs& Q, uint64_t items, uint32_t share,
+                  uint32_t most, cudaStream_t s) {
+    if (r2o)
+        query_dispatch<true>(R, S, Q, items, share, most, s);
+    else
+        query_dispatch<false>(R, S, Q, items, share, most, s);
 }
 
 // Stage B, heavy pass: one warp per spilled candidate.  The warp descends the
@@ -1478,13 +1593,6 @@ __global__ void __launch_bounds__(kHeavyWarps * 32) k_stage_b_heavy(const RobotD
     warp_count(A.stats + 7, n_node);
 }
 
-template <class K>
-static uint32_t grid_for(K kernel, int threads) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
-    return (uint32_t) std::max(1, per_sm) * (uint32_t) device_sm_count();
-}
-
 uint32_t stage_a_blocks(bool r2o) {
     return r2o ? grid_for(k_stage_a<true>, kStageAWarps * 32) : grid_for(k_stage_a<false>, kStageAWarps * 32);
 }
@@ -1556,71 +1664,6 @@ void launch_stage_b_heavy(bool r2o, const RobotDev& R, const SceneDev& S, const 
     else
         k_stage_b_heavy<false><<<hb, kHeavyWarps * 32, 0, s>>>(R, S, W);
     cuda_check(cudaGetLastError(), "k_stage_b_heavy");
-}
-
-// The fused kernel's frontier lives in dynamic shared memory, sized from the
-// scene's wide-tree depth.
-static size_t stage_ab_smem(const SceneDev& S) { return sizeof(uint32_t) * kAbWarps * (size_t) S.wide_front; }
-// with top_nodes wide nodes staged after the frontiers (16-byte aligned)
-static size_t stage_ab_smem(const SceneDev& S, uint32_t top_nodes) {
-    return ((stage_ab_smem(S) + 15) & ~size_t(15)) + (size_t) top_nodes * 2 * kWide * sizeof(float4);
-}
-
-template <class K>
-static uint32_t stage_ab_grid(K kernel, size_t smem) {
-    // beyond the default 48 KB a block needs the opt-in (trees deeper than ~44 wide levels;
-    // the deepest accepted tree needs about 96 KB)
-    if (smem + sizeof(uint32_t) * kAbWarps * kCandBuf > 48 * 1024)
-        cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                   "k_stage_ab shared memory");
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kAbWarps * 32, smem);
-    return (uint32_t) std::max(1, per_sm) * (uint32_t) device_sm_count();
-}
-
-// Runs f with the k_stage_ab instantiation for (r2o, packets, top).
-template <class F>
-static auto with_stage_ab(bool r2o, bool packets, bool top, F&& f) {
-    if (top) {
-        if (packets) return r2o ? f(k_stage_ab<true, true, true>) : f(k_stage_ab<false, true, true>);
-        return r2o ? f(k_stage_ab<true, false, true>) : f(k_stage_ab<false, false, true>);
-    }
-    if (packets) return r2o ? f(k_stage_ab<true, true, false>) : f(k_stage_ab<false, true, false>);
-    return r2o ? f(k_stage_ab<true, false, false>) : f(k_stage_ab<false, false, false>);
-}
-
-uint32_t stage_ab_blocks(bool r2o, bool packets, const SceneDev& S) {
-    const size_t smem = stage_ab_smem(S);
-    return with_stage_ab(r2o, packets, false, [&](auto kernel) { return stage_ab_grid(kernel, smem); });
-}
-
-void launch_subtree(bool r2o, const RobotDev& R, const SceneDev& S, const WaveArgs& W, uint32_t share, cudaStream_t s) {
-    const size_t smem = stage_ab_smem(S);
-    const uint32_t full = r2o ? stage_ab_grid(k_subtree<true, true>, smem) : stage_ab_grid(k_subtree<false, true>, smem);
-    const uint32_t blocks = std::max(1u, full * share / 100);
-    if (r2o) {
-        stage_ab_grid(k_subtree<true, false>, smem);
-        k_subtree<true, true><<<blocks, kAbWarps * 32, smem, s>>>(R, S, W);
-        k_subtree<true, false><<<blocks, kAbWarps * 32, smem, s>>>(R, S, W);
-    } else {
-        stage_ab_grid(k_subtree<false, false>, smem);
-        k_subtree<false, true><<<blocks, kAbWarps * 32, smem, s>>>(R, S, W);
-        k_subtree<false, false><<<blocks, kAbWarps * 32, smem, s>>>(R, S, W);
-    }
-    cuda_check(cudaGetLastError(), "k_subtree");
-}
-
-void launch_stage_ab(bool r2o, bool packets, const RobotDev& R, const SceneDev& S, const WaveArgs& W, uint32_t blocks,
-                     cudaStream_t s) {
-    const uint32_t top = std::min(W.top_nodes, r2o ? S.n_tri_wide : S.n_edge_wide);
-    const size_t smem = stage_ab_smem(S, top);
-    with_stage_ab(r2o, packets, top != 0, [&](auto kernel) {
-        // sets the shared-memory limit before the first launch, and caps the grid at what fits
-        const uint32_t b = std::min(blocks, stage_ab_grid(kernel, smem));
-        kernel<<<b, kAbWarps * 32, smem, s>>>(R, S, W);
-        return 0;
-    });
-    cuda_check(cudaGetLastError(), "k_stage_ab");
 }
 
 uint32_t discrete_persistent_blocks(bool robot_to_obs) {

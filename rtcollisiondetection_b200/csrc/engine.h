@@ -116,6 +116,11 @@ struct WideResult {
     std::vector<float4> cut;
 };
 WideResult build_wide(const float4* d_nodes, uint32_t n_nodes, uint32_t root, DevBuf& out, cudaStream_t s);
+// The same for several trees that share one binary node array (a robot's links): roots[i]'s copy
+// starts at wide node wide_roots[i] (or is the binary root itself when that is kNone or a leaf).
+// Returns the depth of the deepest wide node and the number of nodes (root: unused, no top cut).
+WideResult build_wide_forest(const float4* d_nodes, uint32_t n_nodes, const std::vector<uint32_t>& roots,
+                             std::vector<uint32_t>& wide_roots, DevBuf& out, cudaStream_t s);
 
 // Primitive boxes and gathers (lbvh.cu).
 void tri_boxes(const float* d_verts, const uint32_t* d_tris, uint32_t n, float4* d_lo, float4* d_hi, cudaStream_t s);

@@ -17,6 +17,12 @@ struct RobotDev {
     const float4* edge_prims;       // 2 float4 per edge; w of the first = global edge id
     uint32_t edge_root[kMaxLinks];
     uint32_t n_edges_total;
+    const float4* tri_wide;         // 4-wide copies of the link trees (8 float4 per node), same leaf references
+    uint32_t tri_wide_root[kMaxLinks];   // wide node, or the binary root when that is kNone or a leaf
+    const float4* edge_wide;
+    uint32_t edge_wide_root[kMaxLinks];
+    uint32_t tri_wide_depth, edge_wide_depth;  // deepest wide node of any link
+    uint32_t pair_refs;             // nonzero when every link reference fits beside a candidate's tag
     float4 link_point[kMaxLinks];   // one vertex of each link mesh (link frame)
     const float4* spheres;          // local centre xyz, radius w
     const uint32_t* sphere_link;
@@ -41,12 +47,11 @@ struct SceneDev {
     uint32_t tri_wide_root;   // 0, or the binary root when that is kNone or a leaf
     const float4* edge_wide;
     uint32_t edge_wide_root;
-    uint32_t wide_front;      // frontier entries a warp needs over either wide tree
     const float4* tri_cut;    // top cuts of the wide trees: child records (2 float4 each)
     const float4* edge_cut;
     uint32_t n_tri_cut, n_edge_cut;
     uint32_t edge_wide_lane;  // nonzero when a lane stack of kStack entries holds a wide edge-tree descent
-    uint32_t n_tri_wide, n_edge_wide;  // nodes of the two wide trees
+    uint32_t tri_wide_depth, edge_wide_depth;
 };
 
 struct DiscreteArgs {
@@ -68,13 +73,12 @@ struct DiscreteArgs {
 constexpr int kFkThreads = 128;
 constexpr int kTravThreads = 128;
 
-// Wavefront form of the discrete traversal: stage A (one warp per item)
+// Wavefront form of the discrete traversal (stage_b_form 1, 2): stage A (one warp per item)
 // emits (item position, scene primitive) candidates, stage B (one lane per
 // candidate) runs the link-side descent.  Items whose candidates do not fit
 // the buffer are flagged and re-run by the fused kernel.
 struct WaveArgs {
     DiscreteArgs d;
-    uint32_t top_nodes;        // fused form: wide-tree nodes (from the root) each block stages in shared memory
     uint2* cand;               // (item word pose * n_links + link, scene primitive)
     uint32_t* cand_count;      // zeroed before stage A; may exceed cand_cap
     uint32_t cand_cap;
@@ -82,17 +86,29 @@ struct WaveArgs {
     uint32_t* overflow_items;  // compacted overflowed items (item words, for the fused kernel)
     uint32_t* overflow_count;  // zeroed before stage A
     uint32_t chunk;            // stage B: consecutive candidates (lanes) or 32-candidate groups (packets) per worker
-    uint32_t item_steps;       // fused forms: stage-B steps an item runs in its warp before deferring the rest
     uint32_t light_steps;      // stage B visits before a candidate moves to the heavy pass; 0 = no heavy pass
     uint2* heavy;              // [heavy_cap] candidates (item word, primitive) handed to the heavy pass
     uint32_t heavy_cap;
     uint32_t* heavy_count;     // appended (may exceed heavy_cap: those stayed in the light pass); zeroed
     uint32_t* heavy_work;      // heavy-pass work counter; zeroed
-    uint2* sub;                // [2][sub_cap] (item word, wide node): crowded items' frontiers, then the split pieces
-    uint32_t sub_cap;
-    uint32_t* sub_count;       // [4] zeroed: frontier nodes appended, their work counter, pieces appended, their work
-                               // counter (appends may exceed sub_cap: those items went to the fallback)
 };
+
+// The query kernel: both stages and their load balancing in one launch.
+struct QueryArgs {
+    DiscreteArgs d;
+    unsigned long long* queue;  // low word: tickets taken by idle warps, high word: tasks offered; zeroed
+    uint32_t* live;             // warps of the blocks that have started; zeroed
+    ulonglong2* slot;           // [slots] zeroed: what a ticket's warp gets (see k_query)
+    uint32_t slots;             // a power of two, at least twice the launch's warps
+    uint32_t most_waiting;      // warps that may wait at once; a further idle one leaves
+};
+constexpr uint32_t kQuerySlots = 16384;
+constexpr int kQueryWarps = 4;
+
+// items: an upper bound of the item count; share: percent of the resident grid it
+// may take; most: largest number of blocks.
+void launch_query(bool robot_to_obs, const RobotDev& R, const SceneDev& S, const QueryArgs& Q, uint64_t items,
+                  uint32_t share, uint32_t most, cudaStream_t s);
 
 constexpr int kStageAWarps = 4;
 constexpr int kFrontier = 32 * (kStack + 2);  // bound of a 32-wide LIFO frontier over a tree of depth <= kStack - 2
@@ -107,16 +123,6 @@ void launch_stage_b(bool robot_to_obs, const RobotDev& R, const SceneDev& S, con
 // The heavy pass alone (after a light pass that spilled into W.heavy).
 void launch_stage_b_heavy(bool robot_to_obs, const RobotDev& R, const SceneDev& S, const WaveArgs& W,
                           uint32_t heavy_share, cudaStream_t s);
-// Stages A and B fused in one warp per item (stage_b_form 3; 4 with packet
-// descents of the link tree); spilled candidates go to W.cand / W.heavy.
-void launch_stage_ab(bool robot_to_obs, bool packets, const RobotDev& R, const SceneDev& S, const WaveArgs& W,
-                     uint32_t blocks, cudaStream_t s);
-uint32_t stage_ab_blocks(bool robot_to_obs, bool packets, const SceneDev& S);
-// The subtree pass over the frontiers crowded items handed over (after the
-// fused kernel, before the one-lane pass over the candidates), on share
-// percent of its full persistent grid.
-void launch_subtree(bool robot_to_obs, const RobotDev& R, const SceneDev& S, const WaveArgs& W, uint32_t share,
-                    cudaStream_t s);
 uint32_t stage_a_blocks(bool robot_to_obs);
 uint32_t stage_b_blocks(bool robot_to_obs);
 uint32_t stage_b_max_blocks_per_sm(bool robot_to_obs, uint32_t threads);  // threads: 64, 128 or 256

@@ -555,13 +555,11 @@ static inline float host_u2f(uint32_t u) {
     return f;
 }
 
-WideResult build_wide(const float4* d_nodes, uint32_t n_nodes, uint32_t root, DevBuf& out, cudaStream_t s) {
-    WideResult r;
-    r.root = root;
-    if (root == kNone || (root & kLeaf)) return r;  // empty, or one primitive: no wide nodes
-    std::vector<float4> h(4ull * n_nodes);
-    cuda_check(cudaMemcpyAsync(h.data(), d_nodes, 64ull * n_nodes, cudaMemcpyDeviceToHost, s), "binary nodes download");
-    cuda_check(cudaStreamSynchronize(s), "binary nodes download");
+// Collapses the trees under `roots` (internal binary nodes) into `wide`, breadth-first from all
+// the roots together: root i becomes wide node i.
+static void collapse(const std::vector<float4>& h, const std::vector<uint32_t>& roots, std::vector<float4>& wide,
+                     WideResult& r) {
+    const size_t n_nodes = h.size() / 4;
     struct Kid {
         uint32_t ref;
         float lo[3], hi[3];
@@ -579,8 +577,7 @@ WideResult build_wide(const float4* d_nodes, uint32_t n_nodes, uint32_t root, De
     };
     std::vector<std::pair<uint32_t, uint32_t>> queue;  // (binary node, wide depth)
     queue.reserve(n_nodes / 2 + 1);
-    queue.emplace_back(root, 0u);
-    std::vector<float4> wide;
+    for (uint32_t root : roots) queue.emplace_back(root, 0u);
     wide.reserve(4ull * n_nodes);
     for (size_t qi = 0; qi < queue.size(); ++qi) {
         const uint32_t depth = queue[qi].second;
@@ -619,6 +616,44 @@ WideResult build_wide(const float4* d_nodes, uint32_t n_nodes, uint32_t root, De
         }
     }
     r.nodes = (uint32_t) queue.size();
+}
+
+static std::vector<float4> download_nodes(const float4* d_nodes, uint32_t n_nodes, cudaStream_t s) {
+    std::vector<float4> h(4ull * n_nodes);
+    cuda_check(cudaMemcpyAsync(h.data(), d_nodes, 64ull * n_nodes, cudaMemcpyDeviceToHost, s), "binary nodes download");
+    cuda_check(cudaStreamSynchronize(s), "binary nodes download");
+    return h;
+}
+
+static void upload_wide(const std::vector<float4>& wide, DevBuf& out, cudaStream_t s) {
+    out.ensure(wide.size() * sizeof(float4));
+    cuda_check(cudaMemcpyAsync(out.p, wide.data(), wide.size() * sizeof(float4), cudaMemcpyHostToDevice, s),
+               "wide nodes upload");
+    cuda_check(cudaStreamSynchronize(s), "wide nodes upload");
+}
+
+WideResult build_wide_forest(const float4* d_nodes, uint32_t n_nodes, const std::vector<uint32_t>& roots,
+                             std::vector<uint32_t>& wide_roots, DevBuf& out, cudaStream_t s) {
+    WideResult r;
+    wide_roots = roots;
+    std::vector<uint32_t> inner;
+    for (uint32_t& root : wide_roots)
+        if (root != kNone && !(root & kLeaf)) {
+            inner.push_back(root);
+            root = (uint32_t) inner.size() - 1;
+        }
+    std::vector<float4> wide;
+    if (!inner.empty()) collapse(download_nodes(d_nodes, n_nodes, s), inner, wide, r);
+    if (!wide.empty()) upload_wide(wide, out, s);
+    return r;
+}
+
+WideResult build_wide(const float4* d_nodes, uint32_t n_nodes, uint32_t root, DevBuf& out, cudaStream_t s) {
+    WideResult r;
+    r.root = root;
+    if (root == kNone || (root & kLeaf)) return r;  // empty, or one primitive: no wide nodes
+    std::vector<float4> wide;
+    collapse(download_nodes(d_nodes, n_nodes, s), {root}, wide, r);
     r.root = 0;
     // the top cut: the root's records, each internal one replaced by its node's records, level
     // by level while the list stays within kWideCut records
@@ -645,10 +680,7 @@ WideResult build_wide(const float4* d_nodes, uint32_t n_nodes, uint32_t root, De
         r.cut.push_back(wide[2ull * rec]);
         r.cut.push_back(wide[2ull * rec + 1]);
     }
-    out.ensure(wide.size() * sizeof(float4));
-    cuda_check(cudaMemcpyAsync(out.p, wide.data(), wide.size() * sizeof(float4), cudaMemcpyHostToDevice, s),
-               "wide nodes upload");
-    cuda_check(cudaStreamSynchronize(s), "wide nodes upload");
+    upload_wide(wide, out, s);
     return r;
 }
 

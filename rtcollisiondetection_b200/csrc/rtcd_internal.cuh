@@ -14,18 +14,13 @@ constexpr int kMaxTreeDepth = kStack - 2;  // builders reject deeper trees
 constexpr int kWide = 4;                    // children per node of the scene's wide trees
 constexpr int kWideCut = 64;                // child records in a wide tree's top cut
 
-// Entries a 32-wide LIFO frontier over a kWide-ary tree can hold when every
-// step pops min(size, 32) entries and pushes their internal children, for a
-// tree whose deepest internal node is at depth `depth`: each step's pushes
-// are one segment of at most 32 * kWide entries; the step after it pops 32 of
-// them (or all), so every segment below the top keeps at most
-// 32 * (kWide - 1); and the smallest depth in each live segment exceeds the
-// one below it, so at most depth + 1 segments are live.  A descent that
-// starts from a top cut of at most kWideCut <= 32 * kWide records obeys the
-// same bound.
-__host__ __device__ constexpr uint32_t wide_frontier(uint32_t depth) {
-    return 32u * (kWide - 1) * depth + 32u * kWide;
-}
+// A frontier of fixed size: a step that starts with sp entries pops t of them,
+// at most (cap - reserve - sp) / (kWide - 1) (each popped node adds at most
+// kWide - 1 entries net) but at least one.  With more than one popped the frontier ends at
+// or below cap - reserve; popping one at a time is a depth-first walk, which
+// holds at most kWide - 1 siblings per level above where it began, so a reserve
+// of frontier_reserve(depth) entries is never exceeded.
+__host__ __device__ constexpr uint32_t frontier_reserve(uint32_t depth) { return (kWide - 1) * depth + kWide; }
 
 // device error word bits
 constexpr uint32_t kErrStack = 1u << 0;
