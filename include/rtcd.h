@@ -166,21 +166,13 @@ typedef struct {
                                         group (short trajectories are grouped, long ones staged one at a
                                         time), within the block's share of the SM's shared memory and at
                                         least four groups per resident block (at most 8); 1 = one at a time */
-    uint32_t sweep_heavy_steps;      /* sweeps: frontier steps (each expands up to 32 edge-tree nodes) a heavy-pass
-                                        unit runs before the nodes still open on its frontier (once there are
-                                        four or more) go, one per warp, to a split pass, so a few units with
-                                        very large traversals do not hold the pass while the rest of the GPU
-                                        idles; 0 = 32, 0xFFFFFFFF = never */
+    uint32_t sweep_heavy_steps;      /* accepted, without effect (the heavy pass shares its work as it runs) */
     uint32_t sweep_descend_cap;      /* sweeps, light pass: node visits a lane makes in one descent before the
                                         warp's lanes without work take new units (the descent then resumes
                                         where it stopped), so a lane that finished a short unit does not wait
                                         out a long one; 0 = 3, 0xFFFFFFFF = every descent runs to its next
                                         leaf (the autotuner tries 2, 3, 4 and 6) */
-    uint32_t sweep_heavy_wide;       /* sweeps: 1 = the heavy and split passes expand the scene's 4-wide edge tree,
-                                        four lanes per node (half the levels; faster where many units reach
-                                        the heavy pass near dense geometry), 0 = the binary tree, one lane
-                                        per node (fewer boxes tested: faster on thin geometry); the
-                                        autotuner tries both */
+    uint32_t sweep_heavy_wide;       /* accepted, without effect (the heavy pass descends the 4-wide edge tree) */
 } rtcd_config;
 
 /* Replaces the OptiX context + streams of createContextStream

@@ -497,12 +497,20 @@ struct PlainPool {
     }
 };
 
+// The control block of a check (rtcd_detector.ctl), zeroed by one memset before
+// it: the work counters, the sweep passes' append counters and the counters of
+// the work sharing (share.cuh), each on its own line.
+constexpr size_t kCtlWork = 256, kCtlLive = 384, kCtlOver = 512, kCtlNext = 640, kCtlBytes = 768;
+static_assert(8 * kStatWords <= kCtlWork, "stats overlap the counters");
+
 struct rtcd_detector {
     rtcd_ctx* ctx = nullptr;
     rtcd_detector_kind kind = RTCD_OBS_TO_ROBOT;
     rtcd_robot* robot = nullptr;
     rtcd_scene* scene = nullptr;
     rtcd_config cfg{};
+    unsigned long long* stats() const { return ctl.as<unsigned long long>(); }
+    uint32_t* work() const { return reinterpret_cast<uint32_t*>(ctl.as<uint8_t>() + kCtlWork); }
     std::mutex mu;
     cudaStream_t stream = nullptr;
     cudaEvent_t staged = nullptr;
@@ -517,14 +525,14 @@ struct rtcd_detector {
     bool timed_total_only = false;       // the last check timed only ev[0] -> ev_end (graph path)
     uint32_t blocks = 0;
     // discrete workspace
-    DevBuf q, T, mask, items, count, pose_hit, counts, edge_bits, flags, seg_flags, work, err, stats, contain;
-    DevBuf query;  // the query kernel's queue: counters and slots
+    DevBuf q, T, mask, items, count, pose_hit, counts, edge_bits, flags, seg_flags, err, ctl, contain;
+    DevBuf share;  // the work sharing of a launch: counters and slots
     DevBuf cand, item_overflow, overflow_items, wave_counts;  // wavefront traversal (stage_b_form 1, 2)
     uint32_t blocks_a = 0, blocks_b = 0, blocks_a_full = 0;
     uint32_t threads = 128;  // traversal launch shape (stage B / sweep kernel)
     ScanScratch scan;
     // sweep workspace
-    DevBuf centers, ctrl, aux, piece_hit, W, W_off, heavy, split;
+    DevBuf centers, ctrl, aux, W, W_off, heavy, rest;
     DevBuf edge_q, edge_pose_flags;  // edge checks: interpolated configurations, per-configuration flags
     std::vector<uint32_t> edge_off;
     std::vector<float> W_host;
@@ -967,11 +975,10 @@ rtcd_status rtcd_detector_create(rtcd_ctx* ctx, rtcd_detector_kind kind, rtcd_ro
         }
         apply_launch_shape(d.get());
         d->err.ensure(4);
-        d->stats.ensure(8 * kStatWords);
-        d->work.ensure(32);  // [0] work counter, [1] heavy units appended, [2] heavy-pass counter, [3..4] split pass
+        d->ctl.ensure(kCtlBytes);
         d->count.ensure(4);
         cuda_check(cudaMemset(d->err.p, 0, 4), "memset");
-        cuda_check(cudaMemset(d->stats.p, 0, 8 * kStatWords), "memset");
+        cuda_check(cudaMemset(d->ctl.p, 0, kCtlBytes), "memset");
         if (kind == RTCD_QUAD_SWEEP) ensure_weights(d.get(), kWeightsPrebuilt);
         *out = d.release();
     });
@@ -1182,34 +1189,49 @@ void check_device_errors(rtcd_detector* d, cudaStream_t s) {
     }
 }
 
+// The task queue and the work counter of the next launch on s; `clear` zeroes its
+// counters (a check's first launch finds them zeroed with its control block).
+static TaskQueue task_queue(rtcd_detector* d, bool clear, cudaStream_t s, uint32_t** work_counter) {
+    const size_t slots = sizeof(ulonglong2) * kShareSlots;
+    if (!d->share.p) {
+        d->share.ensure(256 + slots);
+        cuda_check(cudaMemsetAsync(d->share.p, 0, 256, s), "memset");
+        cuda_check(cudaMemsetAsync(d->share.as<uint8_t>() + 256, 0xFF, slots, s), "memset");
+    }
+    uint8_t *base = d->share.as<uint8_t>(), *ctl = d->ctl.as<uint8_t>();
+    if (clear) cuda_check(cudaMemsetAsync(ctl + kCtlLive, 0, kCtlBytes - kCtlLive, s), "memset");
+    TaskQueue q{};
+    q.queue = reinterpret_cast<unsigned long long*>(base);
+    q.live = reinterpret_cast<uint32_t*>(ctl + kCtlLive);
+    q.over = reinterpret_cast<uint32_t*>(ctl + kCtlOver);
+    q.err = d->err.as<uint32_t>();
+    *work_counter = reinterpret_cast<uint32_t*>(ctl + kCtlNext);
+    q.slot = reinterpret_cast<ulonglong2*>(base + 256);
+    q.slots = kShareSlots;
+    q.most_waiting = (uint32_t) device_sm_count();
+    return q;
+}
+
 // One discrete pass over poses [0, n) of d_q.  When `plain`, the item count
 // is read back and the traversal grid sized to it (the upstream shape).
 // The traversal of one direction over the items of the current pass.
 // The first kernel counts into stats bank 0 (and is followed by ev_first,
 // when given), the later passes into bank 1.
-static void traverse(rtcd_detector* d, bool r2o, const DiscreteArgs& A, uint32_t n, bool plain, uint32_t blocks,
-                     uint32_t flags, cudaStream_t s, cudaEvent_t ev_first) {
+static void traverse(rtcd_detector* d, bool r2o, bool first, const DiscreteArgs& A, uint32_t n, bool plain,
+                     uint32_t blocks, uint32_t flags, cudaStream_t s, cudaEvent_t ev_first) {
     RobotDev& R = d->robot->dev;
     const uint32_t L = R.n_links;
     const bool lane_form = d->cfg.stage_b_form == 1 || d->cfg.stage_b_form == 2;
     const uint32_t share = d->cfg.residency_percent ? d->cfg.residency_percent : 100;
     if (!(flags & RTCD_CHECK_FUSED) && !lane_form && R.pair_refs) {
-        const size_t query_bytes = 256 + sizeof(ulonglong2) * kQuerySlots;
-        d->query.ensure(query_bytes);
-        cuda_check(cudaMemsetAsync(d->query.p, 0, query_bytes, s), "memset");
-        uint8_t* base = d->query.as<uint8_t>();
         QueryArgs Q{};
         Q.d = A;
-        Q.d.work_counter = reinterpret_cast<uint32_t*>(base + 128);
-        Q.queue = reinterpret_cast<unsigned long long*>(base);
-        Q.live = reinterpret_cast<uint32_t*>(base + 64);
-        Q.slot = reinterpret_cast<ulonglong2*>(base + 256);
-        Q.slots = kQuerySlots;
+        Q.share = task_queue(d, plain || !first, s, &Q.d.work_counter);
         launch_query(r2o, R, d->scene->dev, Q, (uint64_t) n * (L - R.first_link), share, plain ? blocks : 0xFFFFFFFFu, s);
         if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
         return;
     }
-    cuda_check(cudaMemsetAsync(d->work.p, 0, 8, s), "memset");
+    cuda_check(cudaMemsetAsync(d->work(), 0, 8, s), "memset");
     if ((flags & RTCD_CHECK_FUSED) || !lane_form) {
         launch_discrete(r2o, R, d->scene->dev, A, blocks, s);
         if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
@@ -1244,7 +1266,7 @@ static void traverse(rtcd_detector* d, bool r2o, const DiscreteArgs& A, uint32_t
         W.heavy = d->heavy.as<uint2>();
         W.heavy_cap = hcap;
         W.heavy_count = wc + 3;
-        W.heavy_work = d->work.as<uint32_t>() + 1;
+        W.heavy_work = d->work() + 1;
     }
     const uint32_t ba = plain ? std::max<uint32_t>(1, blocks * kTravThreads / (kStageAWarps * 32)) : d->blocks_a;
     WaveArgs W1 = W;  // the later passes count into bank 1
@@ -1283,7 +1305,7 @@ void discrete_pass(rtcd_detector* d, const float* d_q, uint32_t n, uint32_t* d_h
     if (flags & RTCD_CHECK_NO_CULL) {
         launch_all_items(R, n, d->items.as<uint32_t>(), d->count.as<uint32_t>(), s);
     } else {
-        launch_cull(R, d->scene->dev, d->T.as<float4>(), n, d->mask.as<uint8_t>(), true, d->stats.as<unsigned long long>(),
+        launch_cull(R, d->scene->dev, d->T.as<float4>(), n, d->mask.as<uint8_t>(), true, d->stats(),
                     s);
         select_u8(d->mask.as<uint8_t>(), n * L, d->items.as<uint32_t>(), d->count.as<uint32_t>(), d->scan,
                   d->err.as<uint32_t>(), s);
@@ -1305,9 +1327,9 @@ void discrete_pass(rtcd_detector* d, const float* d_q, uint32_t n, uint32_t* d_h
     A.n_poses = n;
     A.pose_hit = d_hit;
     A.edge_words = (R.n_edges_total + 31) / 32;
-    A.work_counter = d->work.as<uint32_t>();
+    A.work_counter = d->work();
     A.err = d->err.as<uint32_t>();
-    A.stats = d->stats.as<unsigned long long>();
+    A.stats = d->stats();
     A.want_counts = counts ? 1 : 0;
     if (timed) cuda_check(cudaEventRecord(d->ev[2], s), "event");
     const bool own_r2o = d->kind == RTCD_ROBOT_TO_OBS;
@@ -1324,7 +1346,7 @@ void discrete_pass(rtcd_detector* d, const float* d_q, uint32_t n, uint32_t* d_h
         DiscreteArgs Ad = A;
         Ad.counts = (counts && !r2o) ? d_counts : nullptr;
         Ad.edge_bits = (counts && r2o) ? d_bits : nullptr;
-        traverse(d, r2o, Ad, n, plain, blocks, flags, s, timed && k == 0 ? d->ev_first : nullptr);
+        traverse(d, r2o, k == 0, Ad, n, plain, blocks, flags, s, timed && k == 0 ? d->ev_first : nullptr);
         if (counts && r2o) launch_popcount_rows(d_bits, A.edge_words, n, d_counts, s);
     }
     if (d_contain) launch_contain(R, d->scene->dev, A, d_contain, s);
@@ -1535,19 +1557,15 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
                        d->ctrl.as<float4>(), s);
         }
     }
-    d->pose_hit.ensure(4ull * n);
-    cuda_check(cudaMemsetAsync(d->pose_hit.p, 0, 4ull * n, s), "memset");
-    if (want_pieces) {
-        d->piece_hit.ensure(4ull * pieces);
-        cuda_check(cudaMemsetAsync(d->piece_hit.p, 0, 4ull * pieces, s), "memset");
-    }
+    const uint64_t hits = n + (want_pieces ? pieces : 0);  // trajectories, then pieces
+    d->pose_hit.ensure(4ull * hits);
+    cuda_check(cudaMemsetAsync(d->pose_hit.p, 0, 4ull * hits, s), "memset");
     uint32_t* d_counts = nullptr;
     if (counts) {
         d->counts.ensure(4ull * n);
         d_counts = d->counts.as<uint32_t>();
         cuda_check(cudaMemsetAsync(d_counts, 0, 4ull * n, s), "memset");
     }
-    cuda_check(cudaMemsetAsync(d->work.p, 0, 20, s), "memset");  // [0..4]: the sweep passes' counters
     SweepArgs A{};
     A.centers = staged ? nullptr : d->centers.as<float4>();
     A.ctrl = quad && !staged ? d->ctrl.as<float4>() : nullptr;
@@ -1569,37 +1587,34 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
     A.endpoints = !(flags & (RTCD_CHECK_NO_ENDPOINTS | RTCD_CHECK_SURFACE));
     A.surface = (flags & RTCD_CHECK_SURFACE) != 0;
     A.traj_hit = d->pose_hit.as<uint32_t>();
-    A.piece_hit = want_pieces ? d->piece_hit.as<uint32_t>() : nullptr;
+    A.piece_hit = want_pieces ? d->pose_hit.as<uint32_t>() + n : nullptr;
     A.counts = d_counts;
-    A.work_counter = d->work.as<uint32_t>();
+    A.work_counter = d->work();
     A.err = d->err.as<uint32_t>();
-    A.stats = d->stats.as<unsigned long long>();
+    A.stats = d->stats();
     A.want_counts = counts;
     A.want_pieces = want_pieces;
     A.light_steps = d->cfg.light_steps == 0xFFFFFFFFu ? 0u
                     : d->cfg.light_steps                ? d->cfg.light_steps
                                                               : 16u;
-    A.heavy_wide = d->cfg.sweep_heavy_wide ? 1 : 0;
     A.descend_cap = d->cfg.sweep_descend_cap == 0xFFFFFFFFu ? 0u
                     : d->cfg.sweep_descend_cap                ? d->cfg.sweep_descend_cap
                                                                   : 3u;
+    const SceneDev& scene = A.surface && A.total_units ? scene_loop(d->scene) : d->scene->dev;
+    if (scene.n_edges >= (1u << 27)) A.light_steps = 0;  // the heavy pass holds an edge beside a column's tag (wide.cuh)
     if (A.light_steps) {
-        // room for every unit (near dense geometry most units of a piece can spill)
+        // room for every unit (near dense geometry most units of a piece can spill), and for four
+        // open nodes each
         const uint32_t cap = (uint32_t) std::min<uint64_t>(std::max<uint64_t>(pieces * ns, 1024), 1u << 20);
         d->heavy.ensure(sizeof(SweepRec) * cap);
         A.heavy = d->heavy.as<SweepRec>();
         A.heavy_cap = cap;
-        A.heavy_count = d->work.as<uint32_t>() + 1;
-        A.heavy_work = d->work.as<uint32_t>() + 2;
-        // the split pass: room for one frontier entry per unit the light pass could defer
-        A.heavy_steps = d->cfg.sweep_heavy_steps == 0xFFFFFFFFu ? 0u
-                        : d->cfg.sweep_heavy_steps                ? d->cfg.sweep_heavy_steps
-                                                                      : 32u;
-        d->split.ensure(sizeof(uint2) * cap);
-        A.split = d->split.as<uint2>();
-        A.split_cap = cap;
-        A.split_count = d->work.as<uint32_t>() + 3;
-        A.split_work = d->work.as<uint32_t>() + 4;
+        A.heavy_count = d->work() + 1;
+        d->rest.ensure(sizeof(uint2) * 4 * cap);
+        A.rest = d->rest.as<uint2>();
+        A.rest_cap = 4 * cap;
+        A.rest_count = d->work() + 2;
+        A.share = task_queue(d, false, s, &A.rest_work);
     }
     d->last_items = A.total_units;
     if (timed) {
@@ -1608,7 +1623,7 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
     }
     A.binary_tree = d->cfg.stage_b_form == 1 ? 1 : 0;
     if (A.total_units)
-        launch_sweep(A.surface ? scene_loop(d->scene) : d->scene->dev, R, A, d->blocks, d->threads,
+        launch_sweep(scene, R, A, d->blocks, d->threads,
                      d->cfg.residency_percent ? d->cfg.residency_percent : 100, staged, s,
                      timed ? d->ev_first : nullptr);
     else if (timed)
@@ -1616,12 +1631,9 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
     if (timed) cuda_check(cudaEventRecord(d->ev[3], s), "event");
     // outputs
     uint8_t* d_flags = (host || !flags_out) ? (d->flags.ensure(n), d->flags.as<uint8_t>()) : flags_out;
-    launch_flags(d->pose_hit.as<uint32_t>(), n, d_flags, s);
     uint8_t* d_seg = nullptr;
-    if (want_pieces) {
-        d_seg = host ? (d->seg_flags.ensure(pieces), d->seg_flags.as<uint8_t>()) : seg_out;
-        launch_flags(d->piece_hit.as<uint32_t>(), (uint32_t) pieces, d_seg, s);
-    }
+    if (want_pieces) d_seg = host ? (d->seg_flags.ensure(pieces), d->seg_flags.as<uint8_t>()) : seg_out;
+    launch_sweep_flags(d->pose_hit.as<uint32_t>(), n, d_flags, want_pieces ? (uint32_t) pieces : 0, d_seg, s);
     if (host) {
         size_t fpad = (n + 15) & ~15ull, ppad = (pieces + 15) & ~15ull;
         d->pin_out.ensure(fpad + ppad + 4ull * n + 16);
@@ -1656,7 +1668,7 @@ rtcd_status rtcd_check(rtcd_detector* d, const float* q, const uint32_t* traj_of
         d->timed = false;
         d->timed_total_only = false;
         d->last_stream = s;
-        if (n) cuda_check(cudaMemsetAsync(d->stats.p, 0, 8 * kStatWords, s), "stats reset");
+        if (n) cuda_check(cudaMemsetAsync(d->ctl.p, 0, kCtlBytes, s), "control block");
         if (n == 0) return;
         if (flags & RTCD_CHECK_GRAPH) {
             const bool discrete = d->kind == RTCD_OBS_TO_ROBOT || d->kind == RTCD_ROBOT_TO_OBS;
@@ -1825,14 +1837,14 @@ rtcd_status rtcd_last_stats(rtcd_detector* d, rtcd_stats* out) {
         unsigned long long sb[kStatWords] = {0}, st[kStatBank] = {0};
         uint32_t cnt = 0;
         cudaStream_t s = d->last_stream ? d->last_stream : d->stream;
-        cuda_check(cudaMemcpyAsync(sb, d->stats.p, sizeof(sb), cudaMemcpyDeviceToHost, s), "stats");
+        cuda_check(cudaMemcpyAsync(sb, d->stats(), sizeof(sb), cudaMemcpyDeviceToHost, s), "stats");
         cuda_check(cudaMemcpyAsync(&cnt, d->count.p, 4, cudaMemcpyDeviceToHost, s), "stats");
         const bool discrete = d->kind == RTCD_OBS_TO_ROBOT || d->kind == RTCD_ROBOT_TO_OBS;
         uint32_t cand = 0, wave[4] = {0, 0, 0, 0}, work[2] = {0, 0};
         if (d->wave_counts.p)
             cuda_check(cudaMemcpyAsync(wave, d->wave_counts.p, sizeof(wave), cudaMemcpyDeviceToHost, s), "stats");
-        if (!discrete && d->work.p)
-            cuda_check(cudaMemcpyAsync(work, d->work.p, sizeof(work), cudaMemcpyDeviceToHost, s), "stats");
+        if (!discrete)
+            cuda_check(cudaMemcpyAsync(work, d->work(), sizeof(work), cudaMemcpyDeviceToHost, s), "stats");
         cuda_check(cudaStreamSynchronize(s), "stats sync");
         cand = wave[0];
         // the heavy list's append counter: [3] of the discrete wave counters, [1] of the sweep work words
@@ -1978,9 +1990,6 @@ rtcd_status rtcd_detector_autotune(rtcd_detector* d, const float* q_dev, const u
                 c = base;
                 c.sweep_group = base.sweep_group == 1 ? 0u : 1u;
                 time_cfg(c);
-                c = base;
-                c.sweep_heavy_wide = base.sweep_heavy_wide ? 0u : 1u;
-                time_cfg(c);
                 for (uint32_t cap : {2u, 4u, 6u}) {  // visits per descent (0: the default, 3)
                     c = base;
                     c.sweep_descend_cap = base.sweep_descend_cap == cap ? 0u : cap;
@@ -2086,7 +2095,7 @@ rtcd_status rtcd_check_edges(rtcd_detector* d, const float* nodes_dev, uint32_t 
             d->graph_exec = nullptr;
             d->graph = nullptr;
         }
-        cuda_check(cudaMemsetAsync(d->stats.p, 0, 8 * kStatWords, s), "stats reset");
+        cuda_check(cudaMemsetAsync(d->ctl.p, 0, kCtlBytes, s), "control block");
         const uint32_t dof = d->robot->dof;
         const uint32_t total = n_edges * n_wp;
         d->edge_q.ensure(4ull * total * dof);

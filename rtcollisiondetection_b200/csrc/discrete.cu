@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "share.cuh"
 #include "wide.cuh"
 
 namespace cg = cooperative_groups;
@@ -1014,151 +1015,13 @@ static uint32_t grid_for(K kernel, int threads) {
 // memory left 15 of 32 lanes active and handed long descents to passes of
 // their own.)
 //
-// Load balance: a warp that finds the item list empty takes a ticket and waits
-// on that ticket's slot.  A busy warp that sees more tickets taken than tasks
-// offered hands the oldest nodes of its scene frontier, its largest subtrees,
-// to the waiting warps, one each; so the work of one crowded item spreads over
-// the GPU while the others finish, in flag and in count mode alike.  (Pairs and
-// candidates are not handed on: such tasks cost more than they take.)  The warp
-// whose ticket makes every live warp a waiting one ends all of them.  Live are
-// the warps of the blocks that have started: blocks still waiting for room
-// beside another launch's are not waited for, and find the list empty when they
-// come.  A waiting warp gives up after a bounded time; what is offered to a
-// ticket that was given up stays with the warp that offered it, so no task
-// depends on a waiter.
+// Load balance (share.cuh): busy warps hand the oldest nodes of their scene
+// frontier to idle ones, so the work of one crowded item spreads over the GPU
+// while the others finish, in flag and in count mode alike.  (Pairs and
+// candidates are not handed on: such tasks cost more than they take.)
 constexpr int kFrontCap = 512;   // scene nodes waiting (frontier_reserve(kMaxTreeDepth) = 190)
 constexpr int kPairCap = 512;    // (candidate, link node) pairs waiting
 constexpr int kCandBuf = 32 + 32 * kWide;  // < 32 waiting + up to 32 * kWide added by one frontier step
-constexpr int kQueryPolls = 1 << 16;       // polls of a slot (at least 200 ns apart) before a waiting warp gives up
-
-// A slot is two 64-bit words, each with the ticket (plus one) it was written
-// for in its high half, so a reader knows from each word alone whether it is
-// the one it waits for and no fence orders them.  Second word: the scene node.
-// First word: the item, or what became of the ticket.
-constexpr uint32_t kTaken = 0xFFFFFFFFu, kGivenUp = 0xFFFFFFFEu, kOver = 0xFFFFFFFDu;
-__device__ __forceinline__ unsigned long long slot_word(uint32_t t, uint32_t v) {
-    return ((unsigned long long) (t + 1) << 32) | v;
-}
-__device__ __forceinline__ unsigned long long slot_empty(uint32_t t, uint32_t slots) {
-    return t < slots ? 0ull : slot_word(t - slots, kTaken);
-}
-
-// Tickets taken beyond the tasks offered: warps waiting for work.
-__device__ __forceinline__ int waiting(unsigned long long q) { return (int) ((uint32_t) q - (uint32_t) (q >> 32)); }
-
-// Ends the launch when every live warp waits (all lanes call): the tickets taken
-// so far count as served, and their slots are marked.
-__device__ __forceinline__ void end_if_all_wait(const QueryArgs& Q) {
-    const int lane = threadIdx.x & 31;
-    int ended = 0;
-    uint32_t first = 0;
-    if (lane == 0) {
-        __threadfence();  // this warp's ticket, or its leaving, before what it sees of the others
-        for (int tries = 0; tries < 64; ++tries) {
-            const unsigned long long q = *(volatile unsigned long long*) Q.queue;
-            const int waits = waiting(q);
-            if (waits <= 0 || waits < (int) *(volatile uint32_t*) Q.live) break;
-            if (atomicCAS(Q.queue, q, q + ((unsigned long long) waits << 32)) == q) {
-                atomicSub(Q.live, (uint32_t) waits);
-                ended = waits;
-                first = (uint32_t) (q >> 32);
-                break;
-            }
-        }
-    }
-    ended = __shfl_sync(0xffffffffu, ended, 0);
-    first = __shfl_sync(0xffffffffu, first, 0);
-    for (int k = lane; k < ended; k += 32) {
-        const uint32_t i = first + k;
-        atomicCAS(&Q.slot[i & (Q.slots - 1)].x, slot_empty(i, Q.slots), slot_word(i, kOver));
-    }
-    __syncwarp();
-}
-
-// A task for an idle warp (all lanes call): (item, scene node); false when it is
-// to leave: the launch is over, or enough warps wait already (Q.most_waiting).
-__device__ __forceinline__ bool take_task(const QueryArgs& Q, uint2& task) {
-    const int lane = threadIdx.x & 31;
-    uint32_t t = 0, leave = 0;
-    if (lane == 0) {
-        leave = waiting(*(volatile unsigned long long*) Q.queue) >= (int) Q.most_waiting;
-        if (leave) atomicSub(Q.live, 1u);
-        else t = (uint32_t) atomicAdd(Q.queue, 1ull);
-    }
-    leave = __shfl_sync(0xffffffffu, leave, 0);
-    end_if_all_wait(Q);
-    if (leave) return false;
-    uint32_t got = 0;
-    if (lane == 0) {
-        ulonglong2* slot = Q.slot + (t & (Q.slots - 1));
-        uint32_t nap = 100;
-        int polls = 0;
-        unsigned long long w;
-        while (true) {
-            w = *(volatile unsigned long long*) &slot->x;
-            if ((uint32_t) (w >> 32) == t + 1) break;
-            if (++polls > kQueryPolls) {  // gives up, unless a task arrives just now
-                w = atomicCAS(&slot->x, slot_empty(t, Q.slots), slot_word(t, kGivenUp));
-                if ((uint32_t) (w >> 32) != t + 1) atomicSub(Q.live, 1u);
-                break;
-            }
-            __nanosleep(nap);
-            nap = min(2 * nap, 800u);
-        }
-        if ((uint32_t) (w >> 32) == t + 1 && (uint32_t) w < kOver) {
-            task.x = (uint32_t) w;
-            // written before the first word, so it is here or on its way
-            for (polls = 0; polls < kQueryPolls; ++polls) {
-                w = *(volatile unsigned long long*) &slot->y;
-                if ((uint32_t) (w >> 32) == t + 1) break;
-            }
-            task.y = (uint32_t) w;
-            got = 1;
-            atomicExch(&slot->x, slot_word(t, kTaken));
-        }
-    }
-    task.x = __shfl_sync(0xffffffffu, task.x, 0);
-    task.y = __shfl_sync(0xffffffffu, task.y, 0);
-    return __shfl_sync(0xffffffffu, got, 0) != 0;
-}
-
-// Hands up to `want` (at most 32) of the oldest of the scene nodes fr[0, sp) to
-// waiting warps.
-__device__ __forceinline__ void offer_tasks(const QueryArgs& Q, int want, uint32_t item, uint32_t* fr, int& sp) {
-    const int lane = threadIdx.x & 31;
-    const int give = min(want, 32);
-    uint32_t t0 = 0;
-    if (lane == 0) t0 = (uint32_t) (atomicAdd(Q.queue, (unsigned long long) give << 32) >> 32);
-    t0 = __shfl_sync(0xffffffffu, t0, 0);
-    uint32_t node = 0;
-    bool kept = false;
-    if (lane < give) {
-        node = fr[lane];
-        const uint32_t t = t0 + lane;
-        ulonglong2* slot = Q.slot + (t & (Q.slots - 1));
-        const unsigned long long empty = slot_empty(t, Q.slots);
-        // a slot's last user may be about to mark it taken (it has its task): a short, bounded wait
-        for (int polls = 0; polls < 4096; ++polls) {
-            const unsigned long long w = *(volatile unsigned long long*) &slot->x;
-            if (w == empty || w == slot_word(t, kGivenUp)) break;
-        }
-        *(volatile unsigned long long*) &slot->y = slot_word(t, node);
-        kept = atomicCAS(&slot->x, empty, slot_word(t, item)) != empty;
-    }
-    const uint32_t mk_ = __ballot_sync(0xffffffffu, kept);
-    const int back = __popc(mk_);
-    // the nodes kept, then the rest moved down
-    for (int i = 0; i < sp - give; i += 32) {
-        const bool on = i + lane < sp - give;
-        const uint32_t v = on ? fr[give + i + lane] : 0u;
-        __syncwarp();
-        if (on) fr[back + i + lane] = v;
-        __syncwarp();
-    }
-    if (kept) fr[__popc(mk_ & ((1u << lane) - 1u))] = node;
-    sp -= give - back;
-    __syncwarp();
-}
 
 // The OBB test of the scene descents; the warp's box lives in shared memory
 // and is read at every step, so that no register holds it during stage B.
@@ -1177,6 +1040,7 @@ struct ObbTest {
     ObbW ob;
     f3 ext;
     __device__ __forceinline__ explicit ObbTest(const ObbCol& c) : col(c) {}
+    __device__ __forceinline__ bool wants(uint32_t) const { return true; }
     __device__ __forceinline__ void bind(uint32_t) {
         const float4 a = col.v[0], b = col.v[1], c = col.v[2], d = col.v[3], e = col.v[4];
         ob.c = mk(a.x, a.y, a.z);
@@ -1219,6 +1083,7 @@ struct PairTest {
     StageBCand C;
     uint32_t col;
     __device__ __forceinline__ explicit PairTest(const CandCols<R2O>& k) : cols(k) {}
+    __device__ __forceinline__ bool wants(uint32_t) const { return true; }
     __device__ __forceinline__ void bind(uint32_t c) {
         col = c;
         if (R2O) {
@@ -1268,9 +1133,9 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
     const int reserve_b = (int) frontier_reserve(R2O ? R.edge_wide_depth : R.tri_wide_depth);
     const uint32_t n_items = *A.n_items, warps = gridDim.x * kQueryWarps;
     const bool counting = A.want_counts != 0;
-    if (threadIdx.x == 0) s_live = 0;
-    __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(Q.live, (uint32_t) kQueryWarps) != kNone) s_live = 1;  // set once it has returned
+    // blocks beyond the items and the waiting warps have nothing to do
+    if (blockIdx.x * kQueryWarps >= n_items + Q.share.most_waiting) return;
+    share_start(Q.share, &s_live);
     uint32_t n_leaf = 0, n_cand = 0, n_node = 0;
     bool listed = wroot != kNone;  // the item list may hold more
     uint32_t first = blockIdx.x * kQueryWarps + (threadIdx.x >> 5);  // the warp's first item; kNone: taken
@@ -1289,10 +1154,10 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
                 if (n_items - it > warps) poll = 4;
             } else {
                 listed = false;
-                for (int polls = 0; !s_live && polls < kQueryPolls; ++polls) {}  // live before idle
+                share_wait_live(&s_live);
             }
         }
-        if (!listed && !take_task(Q, task)) break;
+        if (!listed && !take_task(Q.share, task)) break;
         const uint32_t item = task.x, pose = item / R.n_links, link = item - pose * R.n_links;
         if (pose >= A.n_poses) {
             if (lane == 0) atomicOr(A.err, kErrRange);
@@ -1301,7 +1166,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
         uint32_t decided = 0;
         if (lane == 0 && !counting) decided = ld_flag(A.pose_hit + pose);
         unsigned long long queue = 0;
-        if (lane == 0) queue = *(volatile unsigned long long*) Q.queue;
+        if (lane == 0) queue = look(Q.share.queue);
         const uint32_t lroot = R2O ? R.edge_wide_root[link] : R.tri_wide_root[link];
         {
             ObbW ob;
@@ -1329,8 +1194,8 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
         if (lane == 0) n_cand += nc;
         auto share = [&](int most) {  // hands up to `most` nodes of the scene frontier to waiting warps
             const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
-            if (want > 0 && most > 0) offer_tasks(Q, min(want, most), item, s.front, sp);
-            if (lane == 0) queue = *(volatile unsigned long long*) Q.queue;
+            if (want > 0 && most > 0) offer_tasks(Q.share, min(want, most), [&](uint32_t) { return item; }, 0xFFFFFFFFu, s.front, sp);
+            if (lane == 0) queue = look(Q.share.queue);
         };
         while (true) {
             if (nc < 32 && sp > 0) {  // stage A
@@ -1459,9 +1324,9 @@ static void query_dispatch(const RobotDev& R, const SceneDev& S, const QueryArgs
     static const uint32_t fit_all = grid_for(k_query<R2O, 5>, kQueryWarps * 32);
     const uint64_t useful = std::max<uint64_t>(2 * sms, items / (Q.d.want_counts ? 4 : 64));
     uint32_t blocks = (uint32_t) std::min<uint64_t>(std::max(1u, (few ? fit_few : fit_all) * share / 100), useful);
-    blocks = std::min({blocks, std::max(1u, most), kQuerySlots / (2 * kQueryWarps)});
+    blocks = std::min({blocks, std::max(1u, most), kShareSlots / (2 * kQueryWarps)});
     QueryArgs G = Q;
-    G.most_waiting = sms;
+    G.share.most_waiting = sms;
     if (few)
         k_query<R2O, 3><<<blocks, kQueryWarps * 32, 0, s>>>(R, S, G);
     else

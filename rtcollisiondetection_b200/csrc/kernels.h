@@ -93,16 +93,24 @@ struct WaveArgs {
     uint32_t* heavy_work;      // heavy-pass work counter; zeroed
 };
 
-// The query kernel: both stages and their load balancing in one launch.
-struct QueryArgs {
-    DiscreteArgs d;
-    unsigned long long* queue;  // low word: tickets taken by idle warps, high word: tasks offered; zeroed
+// Work sharing between the warps of a launch (share.cuh).
+struct TaskQueue {
+    unsigned long long* queue;  // low word: tickets taken by idle warps, high word: tasks offered; equal
+                                // between launches
     uint32_t* live;             // warps of the blocks that have started; zeroed
-    ulonglong2* slot;           // [slots] zeroed: what a ticket's warp gets (see k_query)
+    uint32_t* over;             // set once every live warp waits; zeroed
+    uint32_t* err;              // device error word
+    ulonglong2* slot;           // [slots] what a ticket's warp gets; all ones at first
     uint32_t slots;             // a power of two, at least twice the launch's warps
     uint32_t most_waiting;      // warps that may wait at once; a further idle one leaves
 };
-constexpr uint32_t kQuerySlots = 16384;
+constexpr uint32_t kShareSlots = 32768;
+
+// The query kernel: both stages and their load balancing in one launch.
+struct QueryArgs {
+    DiscreteArgs d;
+    TaskQueue share;
+};
 constexpr int kQueryWarps = 4;
 
 // items: an upper bound of the item count; share: percent of the resident grid it
@@ -139,6 +147,9 @@ void launch_popcount_rows(const uint32_t* d_bits, uint32_t words, uint32_t rows,
 // flags[i] = (hit[i] != 0) | 2 * (contain[i] != 0); contain may be NULL.
 void launch_flags(const uint32_t* d_hit, uint32_t n, uint8_t* d_flags, cudaStream_t s,
                   const uint32_t* d_contain = nullptr);
+// flags[i] = hit[i] != 0 for the n trajectories, seg[i] = hit[n + i] != 0 for the pieces.
+void launch_sweep_flags(const uint32_t* d_hit, uint32_t n, uint8_t* d_flags, uint32_t pieces, uint8_t* d_seg,
+                        cudaStream_t s);
 // Containment of the items' poses not yet hit (sets contain[pose] = 1).
 void launch_contain(const RobotDev& R, const SceneDev& S, const DiscreteArgs& A, uint32_t* d_contain, cudaStream_t s);
 uint32_t discrete_persistent_blocks(bool robot_to_obs);
@@ -180,14 +191,11 @@ struct SweepArgs {
     SweepRec* heavy;           // [heavy_cap] units handed to the heavy pass
     uint32_t heavy_cap;
     uint32_t* heavy_count;     // units appended (may exceed heavy_cap: those stayed in the light pass)
-    uint32_t* heavy_work;      // heavy-pass work counter
-    uint32_t heavy_steps;      // frontier steps a heavy unit takes before its open frontier goes to the split
-                               // pass (0: never)
-    int heavy_wide;            // heavy and split passes on the 4-wide edge tree (else the binary one)
-    uint2* split;              // [split_cap] (heavy record, edge-tree node) pairs for the split pass
-    uint32_t split_cap;
-    uint32_t* split_count;     // pairs appended (past split_cap: the unit was finished by its warp)
-    uint32_t* split_work;      // split-pass work counter
+    uint2* rest;               // [rest_cap] (heavy record, wide edge-tree node): what is left of their descents
+    uint32_t rest_cap;
+    uint32_t* rest_count;      // appended (may exceed rest_cap: those units stayed in the light pass)
+    uint32_t* rest_work;       // heavy-pass work counter
+    TaskQueue share;
     // the staged light pass (k_sweep_traj): a block takes `group` consecutive trajectories at a time
     // from work_counter, runs their FK (and quadratic fit) into shared memory and their units from there
     const float* q;            // [waypoint][dof] joint values

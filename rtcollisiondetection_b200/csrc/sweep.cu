@@ -21,26 +21,28 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "share.cuh"
+#include "wide.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace rtcd {
 
 // ---------------------------------------------------------------- FK + sphere centres
-constexpr int kWpPerBlock = 32;
+constexpr int kWpPerBlock = 32, kFkSphereThreads = 256;
 
-__global__ void __launch_bounds__(kWpPerBlock) k_fk_spheres(const RobotDev R, const float* __restrict__ q, uint32_t n_wp,
+__global__ void __launch_bounds__(kFkSphereThreads) k_fk_spheres(const RobotDev R, const float* __restrict__ q, uint32_t n_wp,
                                                            float4* __restrict__ centers) {
     __shared__ float sT[kWpPerBlock][kMaxLinks][12];
     uint32_t w = blockIdx.x * kWpPerBlock + threadIdx.x;
-    if (w < n_wp) {
+    if (threadIdx.x < kWpPerBlock && w < n_wp) {
         float qq[kMaxDof];
         for (int k = 0; k < R.chain.dof; ++k) qq[k] = q[(size_t) w * R.chain.dof + k];
         fk_chain(R.chain, qq, sT[threadIdx.x]);
     }
     __syncthreads();
     uint32_t nw = min((uint32_t) kWpPerBlock, n_wp - blockIdx.x * kWpPerBlock);
-    for (uint32_t idx = threadIdx.x; idx < nw * R.n_spheres; idx += kWpPerBlock) {
+    for (uint32_t idx = threadIdx.x; idx < nw * R.n_spheres; idx += kFkSphereThreads) {
         uint32_t wl = idx / R.n_spheres, s = idx % R.n_spheres;
         const float* T = sT[wl][R.sphere_link[s]];
         float4 p = R.spheres[s];
@@ -52,7 +54,7 @@ __global__ void __launch_bounds__(kWpPerBlock) k_fk_spheres(const RobotDev R, co
 
 void launch_fk_spheres(const RobotDev& R, const float* d_q, uint32_t n_wp, float4* d_centers, cudaStream_t s) {
     if (!n_wp) return;
-    k_fk_spheres<<<(n_wp + kWpPerBlock - 1) / kWpPerBlock, kWpPerBlock, 0, s>>>(R, d_q, n_wp, d_centers);
+    k_fk_spheres<<<(n_wp + kWpPerBlock - 1) / kWpPerBlock, kFkSphereThreads, 0, s>>>(R, d_q, n_wp, d_centers);
     cuda_check(cudaGetLastError(), "k_fk_spheres");
 }
 
@@ -560,10 +562,11 @@ __device__ __forceinline__ bool leaf_hit_surface(const float4* __restrict__ ep, 
     const float r = U.r, tol = kSweepBand + 1e-6f * r;
     if (!QUAD) {
         const V3<float> a = v3cast<float>(U.P0), b = v3cast<float>(U.P1);
-        const float dseg = sqrtf(fmaxf(seg_seg2<float>(p, q, a, b), 0.f));
-        if (dseg > r + tol) return false;
+        // the cheaper test first: near a capsule most edges start inside it
         const float dp = sqrtf(fmaxf(seg_seg2<float>(p, p, a, b), 0.f));
         if (dp < r - tol) return false;                     // starts inside: never enters
+        const float dseg = sqrtf(fmaxf(seg_seg2<float>(p, q, a, b), 0.f));
+        if (dseg > r + tol) return false;
         if (dseg < r - tol && dp > r + tol) return true;    // a certain hit
     } else {
         const V3<float> B0 = v3cast<float>(U.P0), B1 = v3cast<float>(U.P1), B2 = v3cast<float>(U.P2);
@@ -684,13 +687,29 @@ __device__ __forceinline__ uint32_t sweep_descend(const float4* __restrict__ en,
     return leaf;
 }
 
+// Hands a unit's open descent to the heavy pass: its geometry as a record and
+// each node of the lane's stack as an entry (a descent of the binary tree starts
+// again from the wide tree's root, and its hits are counted there).  False when
+// a list is full: the lane finishes the unit.
+template <bool WIDE>
+__device__ __forceinline__ bool hand_over(const SceneDev& S, const SweepArgs& A, const SweepUnit& U, const uint32_t* st,
+                                          int sp, uint32_t u_hits) {
+    const uint32_t slot = atomicAdd(A.heavy_count, 1u);
+    if (slot >= A.heavy_cap) return false;
+    const uint32_t n = WIDE ? (uint32_t) sp : 1u, base = atomicAdd(A.rest_count, n);
+    const bool fits = (uint64_t) base + n <= A.rest_cap;
+    if (fits) store_rec(A.heavy + slot, U);
+    for (uint32_t k = 0; k < n && (uint64_t) base + k < A.rest_cap; ++k)  // below the capacity every entry is written
+        A.rest[base + k] = fits ? make_uint2(slot, WIDE ? st[k] : S.edge_wide_root) : make_uint2(kNone, kNone);
+    if (fits && WIDE && u_hits) atomicAdd(A.counts + U.traj, u_hits);
+    return fits;
+}
+
 // Light pass: one lane per unit, "while-while" (Aila and Laine 2009): lanes
 // without a unit take their next one, every lane descends to its next leaf,
 // then the warp's leaf tests run together.  A unit still open after
-// A.light_steps node and leaf visits is handed to the heavy pass (its hits
-// so far are set as flags, which are idempotent; its counts are dropped and
-// recounted there), so one lane never serialises a unit that meets thousands
-// of nodes.
+// A.light_steps node and leaf visits is handed to the heavy pass (hand_over),
+// so one lane never serialises a unit that meets thousands of nodes.
 // The quadratic form is capped at 96 registers (5 blocks of 128 threads per
 // SM), the linear one at 80 (6 blocks): the extra resident warps hide more
 // load latency than the few spilled registers cost (measured on the
@@ -769,9 +788,7 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
             }
         }
         if (sp > 0 && steps > budget) {
-            const uint32_t slot = atomicAdd(A.heavy_count, 1u);
-            if (slot < A.heavy_cap) {
-                store_rec(A.heavy + slot, U);
+            if (hand_over<WIDE>(S, A, U, st, sp, u_hits)) {
                 busy = false;
                 continue;
             }
@@ -984,9 +1001,7 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
                 }
             }
             if (sp > 0 && steps > budget) {
-                const uint32_t slot = atomicAdd(A.heavy_count, 1u);
-                if (slot < A.heavy_cap) {
-                    store_rec(A.heavy + slot, U);
+                if (hand_over<WIDE>(S, A, U, st, sp, u_hits)) {
                     busy = false;
                     continue;
                 }
@@ -1005,191 +1020,218 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
     warp_count(A.stats + 7, n_node);
 }
 
-// Heavy pass: one warp per spilled unit.  The warp descends the obstacle-edge
-// LBVH through a shared LIFO frontier (up to 32 nodes a step, survivors
-// pushed), collects leaf survivors in a shared buffer and tests them 32 at a
-// time, one leaf per lane.  The unit's serial depth drops from its node count
-// to about its node count / 32 plus the tree depth.  WIDE: the frontier holds
-// nodes of the scene's 4-wide edge tree instead, up to 8 a step with four
-// lanes per node, each lane loading and testing one child record (half the
-// levels of the binary tree; more boxes tested in all, which the reference's
-// thin shelf boards do not repay: SweepArgs.heavy_wide chooses).
-constexpr int kHeavyWarps = 4;
-constexpr int kLeafBuf = 96;  // < 32 waiting + up to 64 added by one node step
+// Heavy pass: what is left of the descents of the units the light pass handed
+// over, 32 (unit, node) entries a warp at a time.  The units' geometry lies in
+// shared memory, one column per entry, and the warp descends the 4-wide edge
+// tree with all of them at once: its frontier holds (column, node) pairs, lanes
+// take pairs, and the (column, edge) pairs it reaches are tested 32 at a time.
+// Lanes stay busy while any pair waits, and no step waits for one unit's next
+// node.  Without counts a column whose piece (or trajectory) is decided is
+// dropped: at once when this warp decides it, at the next look at the flags
+// otherwise.  Idle warps take pairs of busy ones over (share.cuh), since some
+// units meet tens of thousands of edges.  Every node is expanded exactly once.
+//
+// A warp per unit from the root, and a second launch for the units it did not
+// finish in 32 steps, took 258 us for the 53k open units of 4,096 linear
+// trajectories, 452 us for 45k quadratic ones and 5.2 ms for the 24k of 301
+// trajectories counted over the 202k-triangle shelf; this 116 us, 302 us and
+// 2.3 ms.  Bound by the latency of node and edge loads and, counting, by the
+// 59M edges to test.  More than five (quadratic: three) blocks per SM are
+// slower by up to 6 %.
+constexpr int kRestWarps = 4;
+constexpr int kRestPairs = 512;
+constexpr int kRestLeaf = 32 + 32 * kWide;
 
-// SPLIT = false: the heavy pass over the light pass's deferred units, each
-// from the root.  A unit still open after A.heavy_steps frontier steps, once
-// its frontier holds kSplitMinFront nodes or more, finishes its pending
-// leaves, appends its open frontier nodes to A.split and stops (A.heavy_steps
-// == 0: never), so the few units with very large traversals do not hold the
-// pass while the other warps idle.  SPLIT = true: the split pass, one warp
-// per (unit, node) pair of A.split, each descending that node's subtree to
-// the end.  Every node is expanded exactly once either way, so flags and
-// counts do not depend on where a unit split.
-constexpr int kSplitMinFront = 4;
-template <bool QUAD, bool SURF, bool SPLIT, bool WIDE>
-__global__ void __launch_bounds__(kHeavyWarps * 32) k_sweep_heavy(const SceneDev S, const SweepArgs A) {
-    __shared__ uint32_t s_front[kHeavyWarps][kFrontier];
-    __shared__ uint32_t s_leaf[kHeavyWarps][kLeafBuf];
-    const int lane = threadIdx.x & 31;
-    uint32_t* fr = s_front[threadIdx.x >> 5];
-    uint32_t* lf = s_leaf[threadIdx.x >> 5];
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t n_work = SPLIT ? min(*A.split_count, A.split_cap) : min(*A.heavy_count, A.heavy_cap);
-    unsigned long long n_leaf = 0, n_roots = 0, n_node = 0;
-    while (true) {
-        uint32_t h = 0;
-        if (lane == 0) h = atomicAdd(SPLIT ? A.split_work : A.heavy_work, 1u);
-        h = __shfl_sync(0xffffffffu, h, 0);
-        if (h >= n_work) break;
-        uint32_t rec = h, start = WIDE ? S.edge_wide_root : S.edge_root;
-        if (SPLIT) {
-            const uint2 item = A.split[h];
-            if (item.x == kNone) continue;  // a blanked slot of a reservation that did not fit
-            rec = item.x;
-            start = item.y;
+// The units of a batch in shared memory: [field][column].
+template <bool QUAD>
+struct UnitCols {
+    static constexpr int kCull = QUAD ? 13 : 7;
+    float cull[kCull][32];
+    float geo[QUAD ? 10 : 7][32];  // P0, P1, (P2), r
+    uint32_t rec[32], traj[32], piece[32];
+    __device__ __forceinline__ void put(int c, const SweepUnit& U, uint32_t record) {
+        SweepCull k;
+        make_cull<QUAD>(U, k);
+        for (int a = 0; a < 3; ++a) {
+            cull[a][c] = k.co[a];
+            cull[3 + a][c] = k.cinv[a];
+            if (QUAD) {
+                cull[7 + a][c] = k.blo[a];
+                cull[10 + a][c] = k.bhi[a];
+            }
         }
+        cull[6][c] = k.fat;
+        geo[0][c] = U.P0.x; geo[1][c] = U.P0.y; geo[2][c] = U.P0.z;
+        geo[3][c] = U.P1.x; geo[4][c] = U.P1.y; geo[5][c] = U.P1.z;
+        if (QUAD) {
+            geo[6][c] = U.P2.x; geo[7][c] = U.P2.y; geo[8][c] = U.P2.z;
+        }
+        geo[QUAD ? 9 : 6][c] = U.r;
+        rec[c] = record;
+        traj[c] = U.traj;
+        piece[c] = U.piece_g;
+    }
+    __device__ __forceinline__ SweepUnit unit(uint32_t c) const {
         SweepUnit U;
-        load_rec(A.heavy + rec, U);
-        SweepCull c;
-        make_cull<QUAD>(U, c);
-        if (lane == 0) fr[0] = start;
+        U.P0 = make_float4(geo[0][c], geo[1][c], geo[2][c], 0.f);
+        U.P1 = make_float4(geo[3][c], geo[4][c], geo[5][c], 0.f);
+        U.P2 = QUAD ? make_float4(geo[6][c], geo[7][c], geo[8][c], 0.f) : U.P1;
+        U.r = geo[QUAD ? 9 : 6][c];
+        U.traj = traj[c];
+        U.piece_g = piece[c];
+        return U;
+    }
+};
+
+template <bool QUAD>
+struct UnitTest {
+    const UnitCols<QUAD>& cols;
+    uint32_t alive;  // columns still undecided
+    SweepCull k;
+    __device__ __forceinline__ bool wants(uint32_t c) const { return alive >> c & 1u; }
+    __device__ __forceinline__ void bind(uint32_t c) {
+        for (int a = 0; a < 3; ++a) {
+            k.co[a] = cols.cull[a][c];
+            k.cinv[a] = cols.cull[3 + a][c];
+            if (QUAD) {
+                k.blo[a] = cols.cull[7 + a][c];
+                k.bhi[a] = cols.cull[10 + a][c];
+            }
+        }
+        k.fat = cols.cull[6][c];
+    }
+    __device__ __forceinline__ bool operator()(const Box& b) const {
+        float t;
+        return cull_box<QUAD>(k, b, t);
+    }
+};
+
+template <bool QUAD>
+struct RestWarp {
+    UnitCols<QUAD> cols;
+    uint32_t pairs[kRestPairs];
+    uint32_t leaf[kRestLeaf];
+};
+
+template <bool QUAD, bool SURF>
+__global__ void __launch_bounds__(kRestWarps * 32, QUAD ? 3 : 5) k_sweep_rest(const SceneDev S, const SweepArgs A) {
+    __shared__ RestWarp<QUAD> s_warp[kRestWarps];
+    __shared__ volatile uint32_t s_live;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    RestWarp<QUAD>& s = s_warp[threadIdx.x >> 5];
+    const uint32_t n_rest = min(*A.rest_count, A.rest_cap), warps = gridDim.x * kRestWarps;
+    // entries a warp takes at a time: about four turns each, so that a short list uses every warp
+    const uint32_t per = max(1u, min(32u, n_rest / (4 * warps)));
+    // blocks beyond the list and the waiting warps have nothing to do
+    if ((uint64_t) blockIdx.x * kRestWarps * per >= (uint64_t) n_rest + (uint64_t) A.share.most_waiting * per) return;
+    const int reserve = (int) frontier_reserve(S.edge_wide_depth);
+    const bool counting = A.want_counts != 0;
+    share_start(A.share, &s_live);
+    uint32_t n_leaf = 0, n_node = 0;
+    unsigned long long n_roots = 0;
+    bool listed = true;
+    uint32_t first = blockIdx.x * kRestWarps + (threadIdx.x >> 5);  // the warp's first turn; kNone: taken
+    while (true) {
+        uint2 task = make_uint2(kNone, 0u);  // this lane's (record, node)
+        if (listed) {
+            uint32_t e = first;
+            if (e == kNone) {
+                if (lane == 0) e = warps + atomicAdd(A.rest_work, 1u);
+                e = __shfl_sync(0xffffffffu, e, 0);
+            }
+            first = kNone;
+            e = min(e, n_rest) * per;
+            if (e < n_rest) {
+                if (lane < per && e + lane < n_rest) task = A.rest[e + lane];
+            } else {
+                listed = false;
+                share_wait_live(&s_live);
+            }
+        }
+        if (!listed) {
+            if (!take_task(A.share, task)) break;
+            if (lane > 0) task.x = kNone;
+        }
+        unsigned long long queue = 0;
+        if (lane == 0) queue = look(A.share.queue);
+        bool on = task.x != kNone;  // not a blank of a reservation that did not fit
+        const uint32_t* flag = nullptr;
+        uint32_t decided = 0;
+        if (on) {
+            SweepUnit U;
+            load_rec(A.heavy + task.x, U);
+            flag = A.want_pieces ? A.piece_hit + U.piece_g : A.traj_hit + U.traj;
+            on = counting || !ldflag(flag);
+            s.cols.put(lane, U, task.x);
+        }
+        const uint32_t mon = __ballot_sync(0xffffffffu, on);
+        const bool leaf0 = on && (task.y & kLeaf), node0 = on && !leaf0;
+        const uint32_t ml = __ballot_sync(0xffffffffu, leaf0), mn = __ballot_sync(0xffffffffu, node0);
+        const uint32_t tag = (uint32_t) lane << kTagShift;
+        if (leaf0) s.leaf[__popc(ml & lt)] = tag | (task.y & ~kLeaf);
+        if (node0) s.pairs[__popc(mn & lt)] = tag | task.y;
+        int np = __popc(mn), nl = __popc(ml);
         __syncwarp();
-        int sp = 1, nl = 0, step = 0;
-        uint32_t hits = 0, warp_steps = 0;
-        bool budgeted = !SPLIT && A.heavy_steps != 0, handing = false;
-        while (true) {
-            if (nl >= 32 || (sp == 0 && nl > 0) || (handing && nl > 0)) {  // leaf step
-                const int take = min(nl, 32);
-                nl -= take;
-                const uint32_t leaf = lane < take ? lf[nl + lane] : kNone;
-                __syncwarp();
-                bool hit = false;
-                if (leaf != kNone) {
-                    ++n_leaf;
-                    hit = SURF ? leaf_hit_surface<QUAD>(S.edge_prims, leaf, U, A.stats, n_roots)
-                               : leaf_hit<QUAD>(S.edge_prims, leaf, U, A.stats, n_roots);
-                }
-                const uint32_t mh = __ballot_sync(0xffffffffu, hit);
-                if (mh) {
-                    if (lane == 0) {
-                        if (A.want_pieces) atomicExch(A.piece_hit + U.piece_g, 1u);
-                        if (A.want_counts) {
-                            A.traj_hit[U.traj] = 1u;
-                            hits += __popc(mh);
-                        } else {
-                            atomicExch(A.traj_hit + U.traj, 1u);
-                        }
+        UnitTest<QUAD> test{s.cols, mon};
+        uint32_t tick = 0;
+        while (test.alive) {
+            if (nl < 32 && np > 0) {
+                if ((++tick & (QUAD ? 0 : 3)) == 0) {
+                    const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
+                    if (want > 0 && np > 1)
+                        offer_tasks(A.share, min(want, np >> 1), [&](uint32_t e) { return s.cols.rec[e >> kTagShift]; },
+                                    kTagRef, s.pairs, np);
+                    if (lane == 0) queue = look(A.share.queue);
+                    if (!counting) {  // the flags read at the last look, and read again for the next
+                        test.alive &= __ballot_sync(0xffffffffu, decided == 0);
+                        if (on) decided = ldflag(flag);
                     }
-                    if (!A.want_counts) break;
                 }
+                if (!frontier_step<true>(S.edge_wide, s.pairs, np, s.leaf, nl, test, kRestPairs, reserve, A.err, n_node)) break;
                 continue;
             }
-            if (sp == 0) break;
-            if (handing) {  // no leaves pending: the open frontier goes to the split pass
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(A.split_count, (uint32_t) sp);
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if ((uint64_t) base + (uint64_t) sp <= A.split_cap) {
-                    for (int k = lane; k < sp; k += 32) A.split[base + k] = make_uint2(rec, fr[k]);
-                    break;
+            if (nl == 0) break;
+            const int some = min(nl, 32);
+            nl -= some;
+            bool hit = false;
+            uint32_t c = 0;
+            if (lane < some) {
+                const uint32_t e = s.leaf[nl + lane];
+                c = e >> kTagShift;
+                if (test.wants(c)) {
+                    const SweepUnit U = s.cols.unit(c);
+                    ++n_leaf;
+                    hit = SURF ? leaf_hit_surface<QUAD>(S.edge_prims, e & kTagRef, U, A.stats, n_roots)
+                               : leaf_hit<QUAD>(S.edge_prims, e & kTagRef, U, A.stats, n_roots);
                 }
-                // no room: this warp finishes the unit, and the reserved slots below the capacity
-                // are blanked (the split pass reads every slot up to it)
-                for (int k = lane; k < sp && (uint64_t) base + (uint64_t) k < A.split_cap; k += 32)
-                    A.split[base + k] = make_uint2(kNone, kNone);
-                handing = false;
-                budgeted = false;
             }
-            if (budgeted && ++warp_steps >= A.heavy_steps && sp >= kSplitMinFront) {
-                handing = true;
-                continue;
-            }
-            if (!A.want_counts && (++step & 7) == 0) {  // decided meanwhile by another unit?
-                uint32_t dec = 0;
-                if (lane == 0) dec = A.want_pieces ? ldflag(A.piece_hit + U.piece_g) : ldflag(A.traj_hit + U.traj);
-                if (__shfl_sync(0xffffffffu, dec, 0)) break;
-            }
-            if constexpr (WIDE) {
-                // up to 8 wide nodes a step, four lanes per node, one child record per lane
-                const int take = min(sp, 32 / kWide);
-                sp -= take;
-                const int slot = lane / kWide, j = lane % kWide;
-                const uint32_t ref = slot < take ? fr[sp + slot] : kNone;
-                __syncwarp();
-                bool hc = false;
-                uint32_t rc = kNone;
-                if (ref != kNone) {
-                    if (ref & kLeaf) {  // a one-edge scene: the root itself is a leaf
-                        if (j == 0) {
-                            hc = true;
-                            rc = ref;
+            const uint32_t mh = __ballot_sync(0xffffffffu, hit);
+            if (mh) {
+                if (hit) {
+                    const uint32_t tr = s.cols.traj[c];
+                    if (counting) {
+                        const uint32_t same = __match_any_sync(mh, tr);
+                        if (lane == __ffs(same) - 1) {
+                            atomicAdd(A.counts + tr, (uint32_t) __popc(same));
+                            A.traj_hit[tr] = 1u;
                         }
                     } else {
-                        const float4* r = S.edge_wide + 2ull * kWide * ref + 2 * j;
-                        const float4 ra = __ldg(r), rb = __ldg(r + 1);
-                        rc = __float_as_uint(rb.z);
-                        if (rc != kNone) {  // an empty slot of a node with fewer than four children
-                            ++n_node;
-                            Box bx;
-                            bx.lo[0] = ra.x; bx.lo[1] = ra.y; bx.lo[2] = ra.z;
-                            bx.hi[0] = ra.w; bx.hi[1] = rb.x; bx.hi[2] = rb.y;
-                            float t;
-                            hc = cull_box<QUAD>(c, bx, t);
-                        }
+                        atomicExch(A.traj_hit + tr, 1u);
+                    }
+                    if (A.want_pieces) atomicExch(A.piece_hit + s.cols.piece[c], 1u);
+                }
+                if (!counting) {  // every column of a piece (trajectory) just hit is decided
+                    const uint32_t own = A.want_pieces ? s.cols.piece[lane] : s.cols.traj[lane];
+                    for (uint32_t m = mh; m; m &= m - 1) {
+                        const uint32_t hc = __shfl_sync(0xffffffffu, c, __ffs(m) - 1);
+                        const uint32_t key = A.want_pieces ? s.cols.piece[hc] : s.cols.traj[hc];
+                        test.alive &= ~__ballot_sync(0xffffffffu, own == key);
                     }
                 }
-                const bool pc = hc && !(rc & kLeaf), ec = hc && (rc & kLeaf);
-                const uint32_t mpc = __ballot_sync(0xffffffffu, pc), mec = __ballot_sync(0xffffffffu, ec);
-                const int npush = __popc(mpc);
-                if (sp + npush > kFrontier) {  // cannot happen for trees within the depth limit
-                    if (lane == 0) atomicOr(A.err, kErrStack);
-                    break;
-                }
-                if (pc) fr[sp + __popc(mpc & lt)] = rc;
-                sp += npush;
-                if (ec) lf[nl + __popc(mec & lt)] = rc & ~kLeaf;
-                nl += __popc(mec);
-                __syncwarp();
-                continue;
             }
-            const int take = min(sp, 32);
-            sp -= take;
-            const uint32_t ref = lane < take ? fr[sp + lane] : kNone;
-            __syncwarp();
-            bool hl = false, hr = false;
-            uint32_t rl = kNone, rr = kNone;
-            if (ref != kNone) {
-                if (ref & kLeaf) {  // a one-edge scene: the root itself is a leaf
-                    hl = true;
-                    rl = ref;
-                } else {
-                    Box bl, br;
-                    float t;
-                    load_node(S.edge_nodes, ref, bl, br, rl, rr);
-                    n_node += 2;
-                    hl = cull_box<QUAD>(c, bl, t);
-                    hr = cull_box<QUAD>(c, br, t);
-                }
-            }
-            const bool pl = hl && !(rl & kLeaf), pr = hr && !(rr & kLeaf);
-            const bool el = hl && (rl & kLeaf), er = hr && (rr & kLeaf);
-            const uint32_t mpl = __ballot_sync(0xffffffffu, pl), mpr = __ballot_sync(0xffffffffu, pr);
-            const uint32_t mel = __ballot_sync(0xffffffffu, el), mer = __ballot_sync(0xffffffffu, er);
-            const int npush = __popc(mpl) + __popc(mpr);
-            if (sp + npush > kFrontier) {  // cannot happen for trees within the depth limit
-                if (lane == 0) atomicOr(A.err, kErrStack);
-                break;
-            }
-            if (pl) fr[sp + __popc(mpl & lt)] = rl;
-            if (pr) fr[sp + __popc(mpl) + __popc(mpr & lt)] = rr;
-            sp += npush;
-            if (el) lf[nl + __popc(mel & lt)] = rl & ~kLeaf;
-            if (er) lf[nl + __popc(mel) + __popc(mer & lt)] = rr & ~kLeaf;
-            nl += __popc(mel) + __popc(mer);
             __syncwarp();
         }
-        if (lane == 0 && hits) atomicAdd(A.counts + U.traj, hits);
         __syncwarp();
     }
     warp_count(A.stats + 4, n_leaf);
@@ -1255,17 +1297,6 @@ uint32_t sweep_max_blocks_per_sm(bool quad, uint32_t threads) {
 
 uint32_t sweep_persistent_blocks(bool quad) { return sweep_max_blocks_per_sm(quad, kTravThreads) * device_sm_count(); }
 
-template <bool QUAD, bool SURF, bool WIDE>
-static uint32_t heavy_blocks() {
-    static uint32_t blocks = 0;
-    if (!blocks) {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_heavy<QUAD, SURF, false, WIDE>, kHeavyWarps * 32, 0);
-        blocks = (uint32_t) std::max(1, per_sm) * device_sm_count();
-    }
-    return blocks;
-}
-
 // The staged light pass at BLOCK threads per block, `slot` bytes of shared
 // memory per trajectory, on at most as many blocks as fit.  Trajectories per
 // group (A.group, 0 = chosen here): about 1,024 (piece, sphere) units a
@@ -1321,17 +1352,17 @@ static void launch_staged(const SceneDev& S, const RobotDev& R, const SweepArgs&
     kern<<<blocks, BLOCK, smem, s>>>(S, R, G);
 }
 
-// The heavy pass over the light pass's deferred units, then (A.heavy_steps)
-// the split pass over the frontier nodes the heavy pass handed on.
-template <bool QUAD, bool SURF, bool WIDE>
+// The heavy pass over what the light pass handed over.
+template <bool QUAD, bool SURF>
 static void launch_heavy(const SceneDev& S, const SweepArgs& H, uint32_t heavy_share, cudaStream_t s) {
-    const uint32_t hb = std::max(1u, heavy_blocks<QUAD, SURF, WIDE>() * heavy_share / 100);
-    k_sweep_heavy<QUAD, SURF, false, WIDE><<<hb, kHeavyWarps * 32, 0, s>>>(S, H);
-    cuda_check(cudaGetLastError(), "k_sweep_heavy");
-    if (H.heavy_steps) {
-        k_sweep_heavy<QUAD, SURF, true, WIDE><<<hb, kHeavyWarps * 32, 0, s>>>(S, H);
-        cuda_check(cudaGetLastError(), "k_sweep_heavy (split)");
-    }
+    static const uint32_t full = [] {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_rest<QUAD, SURF>, kRestWarps * 32, 0);
+        return (uint32_t) std::max(1, per_sm) * (uint32_t) device_sm_count();
+    }();
+    const uint32_t blocks = std::min(std::max(1u, full * heavy_share / 100), kShareSlots / (2 * kRestWarps));
+    k_sweep_rest<QUAD, SURF><<<blocks, kRestWarps * 32, 0, s>>>(S, H);
+    cuda_check(cudaGetLastError(), "k_sweep_rest");
 }
 
 template <bool QUAD, bool SURF>
@@ -1369,9 +1400,23 @@ static void sweep_dispatch(const SceneDev& S, const RobotDev& R, const SweepArgs
     if (A.light_steps) {
         SweepArgs H = A;
         H.stats = A.stats + kStatBank;
-        if (A.heavy_wide) launch_heavy<QUAD, SURF, true>(S, H, heavy_share, s);
-        else launch_heavy<QUAD, SURF, false>(S, H, heavy_share, s);
+        launch_heavy<QUAD, SURF>(S, H, heavy_share, s);
     }
+}
+
+__global__ void k_sweep_flags(const uint32_t* __restrict__ hit, uint32_t n, uint8_t* __restrict__ flags, uint32_t pieces,
+                              uint8_t* __restrict__ seg) {
+    const uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
+    if (i < n) flags[i] = hit[i] != 0;
+    else if (i - n < pieces) seg[i - n] = hit[i] != 0;
+}
+
+void launch_sweep_flags(const uint32_t* d_hit, uint32_t n, uint8_t* d_flags, uint32_t pieces, uint8_t* d_seg,
+                        cudaStream_t s) {
+    const uint64_t total = (uint64_t) n + pieces;
+    if (!total) return;
+    k_sweep_flags<<<(uint32_t) ((total + 255) / 256), 256, 0, s>>>(d_hit, n, d_flags, pieces, d_seg);
+    cuda_check(cudaGetLastError(), "k_sweep_flags");
 }
 
 void launch_sweep(const SceneDev& S, const RobotDev& R, const SweepArgs& A, uint32_t blocks, uint32_t threads,

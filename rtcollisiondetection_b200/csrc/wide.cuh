@@ -69,10 +69,10 @@ __device__ __forceinline__ bool frontier_step(const float4* __restrict__ wn, uin
     const int take = min(min(sp, 32 >> lg), max(1, (cap - reserve - sp) / (kWide - 1)));
     sp -= take;
     const int j = lane >> lg;
-    const bool on = j < take;
-    const uint32_t entry = on ? fr[sp + j] : 0u;
+    const uint32_t entry = j < take ? fr[sp + j] : 0u;
     const uint32_t node = TAGGED ? entry & kTagRef : entry;
     const uint32_t tag = TAGGED ? entry & ~kTagRef : 0u;
+    const bool on = j < take && test.wants(tag >> kTagShift);  // an entry nobody wants any more is dropped
     __syncwarp();
     const int rounds = kWide >> lg;
     const float4* rec = wn + 2ull * (kWide * (size_t) node + (lane & (g - 1)));
