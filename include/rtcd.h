@@ -63,9 +63,8 @@ typedef enum {
                                               memory (cudaHostAlloc, cudaHostRegister) is uploaded by DMA
                                               directly, pageable memory is copied into the detector's pinned
                                               staging first */
-#define RTCD_CHECK_NO_CULL (1u << 2)       /* skip the OBB prefilter of the discrete detectors (every item goes to
-                                              the traversal, whose first step rejects the far ones: up to 9 % faster at
-                                              a few thousand poses, slower at tens of thousands) */
+#define RTCD_CHECK_NO_CULL (1u << 2)       /* skip the prefilter of the discrete detectors (every item goes to the
+                                              traversal, whose first step rejects the far ones) */
 #define RTCD_CHECK_PLAIN (1u << 3)         /* discrete: the upstream check() shape - frames of frame_size poses over
                                               plain_streams streams, one host thread per stream, a host round trip
                                               per frame (the culled item count) and a wait after every group of

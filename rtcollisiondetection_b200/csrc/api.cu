@@ -343,6 +343,78 @@ std::vector<uint32_t> loop_edges(const uint32_t* tris, size_t n_tris) {
     return out;
 }
 
+// Spheres that together hold every triangle and edge of a link, appended as
+// (centre, radius): its OBB is cut into about kCoverCells near-cubic cells, and
+// each cell with a primitive's centroid gets the sphere around the box of its
+// primitives' vertices (in the OBB's axes), grown by 1e-4 m.
+constexpr int kCoverCells = 24;
+
+static void cover_spheres(const float* verts, const uint32_t* tris, size_t n_tris, const uint32_t* edges, size_t n_edges,
+                          const float* obb, std::vector<float>& out) {
+    const float* h = obb + 3;
+    float size = std::cbrt(std::max(8.0f * h[0] * h[1] * h[2], 1e-12f) / kCoverCells);
+    size = std::max(size, 2.0f * std::max(h[0], std::max(h[1], h[2])) / kCoverCells);  // a thin box: not more along it
+    int dim[3];
+    for (int k = 0; k < 3; ++k) dim[k] = std::min(kCoverCells, std::max(1, (int) std::lround(2.0f * h[k] / size)));
+    struct Cell {
+        bool used = false;
+        float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f}, r2 = 0.f;
+    };
+    std::vector<Cell> cells((size_t) dim[0] * dim[1] * dim[2]);
+    auto local = [&](uint32_t v, float* x) {  // in the OBB's axes, from its centre
+        const float d[3] = {verts[3ull * v] - obb[0], verts[3ull * v + 1] - obb[1], verts[3ull * v + 2] - obb[2]};
+        for (int k = 0; k < 3; ++k) x[k] = d[0] * obb[6 + 3 * k] + d[1] * obb[7 + 3 * k] + d[2] * obb[8 + 3 * k];
+    };
+    auto cell_of = [&](const uint32_t* idx, int m) -> Cell& {
+        float c[3] = {0, 0, 0};
+        for (int j = 0; j < m; ++j) {
+            float x[3];
+            local(idx[j], x);
+            for (int k = 0; k < 3; ++k) c[k] += x[k] / m;
+        }
+        size_t at = 0;
+        for (int k = 2; k >= 0; --k) {
+            const float t = h[k] > 0 ? (c[k] + h[k]) / (2.0f * h[k]) * dim[k] : 0.f;
+            at = at * dim[k] + (size_t) std::min((float) (dim[k] - 1), std::max(0.0f, t));
+        }
+        return cells[at];
+    };
+    auto each = [&](auto&& f) {
+        for (size_t i = 0; i < n_tris; ++i) f(tris + 3 * i, 3);
+        for (size_t i = 0; i < n_edges; ++i) f(edges + 2 * i, 2);
+    };
+    each([&](const uint32_t* idx, int m) {
+        Cell& c = cell_of(idx, m);
+        c.used = true;
+        for (int j = 0; j < m; ++j) {
+            float x[3];
+            local(idx[j], x);
+            for (int k = 0; k < 3; ++k) {
+                c.lo[k] = std::min(c.lo[k], x[k]);
+                c.hi[k] = std::max(c.hi[k], x[k]);
+            }
+        }
+    });
+    each([&](const uint32_t* idx, int m) {
+        Cell& c = cell_of(idx, m);
+        for (int j = 0; j < m; ++j) {
+            float x[3], r2 = 0.f;
+            local(idx[j], x);
+            for (int k = 0; k < 3; ++k) r2 += (x[k] - 0.5f * (c.lo[k] + c.hi[k])) * (x[k] - 0.5f * (c.lo[k] + c.hi[k]));
+            c.r2 = std::max(c.r2, r2);
+        }
+    });
+    for (const Cell& c : cells) {
+        if (!c.used) continue;
+        for (int a = 0; a < 3; ++a) {
+            float v = obb[a];
+            for (int k = 0; k < 3; ++k) v += 0.5f * (c.lo[k] + c.hi[k]) * obb[6 + 3 * k + a];
+            out.push_back(v);
+        }
+        out.push_back(std::sqrt(c.r2) * 1.0001f + 1e-4f);
+    }
+}
+
 // Device LBVH over triangles or edges, concatenated over several groups
 // (links); returns per-group roots.
 struct GroupedBvh {
@@ -409,6 +481,7 @@ struct rtcd_robot {
     RobotDev dev{};
     GroupedBvh tri, edge;
     DevBuf tri_wide, edge_wide;  // 4-wide copies of the link trees
+    DevBuf cover;                // covering spheres (RobotDev.cover)
     DevBuf verts, tris, edges, spheres, sphere_link;
     std::vector<uint32_t> edge_off;
     uint32_t dof = 0;
@@ -418,7 +491,7 @@ struct rtcd_scene {
     rtcd_ctx* ctx = nullptr;
     SceneDev dev{};
     GroupedBvh tri, edge;
-    DevBuf verts, tris, edges, obbs, tri_obs, obs_box, obs_point;
+    DevBuf verts, tris, edges, obbs, tri_obs, obs_box, obs_point, clear;
     DevBuf tri_wide, edge_wide, tri_cut, edge_cut;  // 4-wide copies of the two scene trees and their top cuts
     uint32_t n_tris = 0, n_edges = 0, n_obs = 0;
     // the directed loop edges and their trees, built on the first surface-semantics sweep
@@ -498,9 +571,9 @@ struct PlainPool {
 };
 
 // The control block of a check (rtcd_detector.ctl), zeroed by one memset before
-// it: the work counters, the sweep passes' append counters and the counters of
-// the work sharing (share.cuh), each on its own line.
-constexpr size_t kCtlWork = 256, kCtlLive = 384, kCtlOver = 512, kCtlNext = 640, kCtlBytes = 768;
+// it: the work counters, the sweep passes' append counters, the counters of the
+// work sharing (share.cuh), each on its own line, and k_prepare's list lengths.
+constexpr size_t kCtlWork = 256, kCtlLive = 384, kCtlOver = 512, kCtlNext = 640, kCtlLinks = 768, kCtlBytes = 832;
 static_assert(8 * kStatWords <= kCtlWork, "stats overlap the counters");
 
 struct rtcd_detector {
@@ -525,7 +598,7 @@ struct rtcd_detector {
     bool timed_total_only = false;       // the last check timed only ev[0] -> ev_end (graph path)
     uint32_t blocks = 0;
     // discrete workspace
-    DevBuf q, T, mask, items, count, pose_hit, counts, edge_bits, flags, seg_flags, err, ctl, contain;
+    DevBuf q, T, mask, items, lists, count, pose_hit, counts, edge_bits, flags, seg_flags, err, ctl, contain;
     DevBuf share;  // the work sharing of a launch: counters and slots
     DevBuf cand, item_overflow, overflow_items, wave_counts;  // wavefront traversal (stage_b_form 1, 2)
     uint32_t blocks_a = 0, blocks_b = 0, blocks_a_full = 0;
@@ -541,6 +614,7 @@ struct rtcd_detector {
     HostBuf pin_in, pin_out, pin_aux;
     DevBuf hq, hflags, hseg, hcounts;  // device sides of a graph replay with host buffers
     uint64_t last_items = 0, last_culled = 0;
+    bool last_lists = false;       // the last check's items are k_prepare's lists
     uint32_t last_path_flags = 0;  // rtcd_stats.path_flags of the last check
     // plain path: one clone of this detector per stream (own stream and workspace) and their threads
     std::vector<rtcd_detector*> plain_clones;
@@ -740,7 +814,16 @@ rtcd_status rtcd_robot_create(rtcd_ctx* ctx, const rtcd_robot_desc* d, rtcd_robo
                 fit_obb(d->link_verts, idx, 1e-5f, o);
             }
         }
+        std::vector<float> cover;
+        for (uint32_t l = 0; l < L; ++l) {
+            r->dev.cover_off[l] = (uint32_t) cover.size() / 4;
+            cover_spheres(d->link_verts + 3ull * voff[l], d->link_tris + 3ull * toff[l], toff[l + 1] - toff[l],
+                          edges.data() + 2ull * eoff[l], eoff[l + 1] - eoff[l], r->dev.obb[l], cover);
+        }
+        for (uint32_t l = L; l <= (uint32_t) kMaxLinks; ++l) r->dev.cover_off[l] = (uint32_t) cover.size() / 4;
         cudaStream_t s = ctx->stream;
+        upload(r->cover, cover.data(), cover.size(), s);
+        r->dev.cover = r->cover.as<float4>();
         upload(r->verts, d->link_verts, 3ull * voff[L], s);
         upload(r->tris, d->link_tris, 3ull * toff[L], s);
         upload(r->edges, edges.data(), edges.size(), s);
@@ -880,6 +963,13 @@ rtcd_status rtcd_scene_create(rtcd_ctx* ctx, const float* verts, uint32_t n_vert
         const WideResult we =
             build_wide(sc->edge.nodes.as<float4>(), node_count(sc->n_edges), sc->edge.roots[0], sc->edge_wide, s);
         SceneDev& dv = sc->dev;
+        float box_lo[3] = {3e38f, 3e38f, 3e38f}, box_hi[3] = {-3e38f, -3e38f, -3e38f};
+        for (uint32_t o = 0; o < nob; ++o)
+            for (int a = 0; a < 3 && off[o + 1] > off[o]; ++a) {
+                box_lo[a] = std::min(box_lo[a], obs_box[8ull * o + a]);
+                box_hi[a] = std::max(box_hi[a], obs_box[8ull * o + 4 + a]);
+            }
+        build_clearance(sc->verts.as<float>(), sc->tris.as<uint32_t>(), n_tris, box_lo, box_hi, sc->clear, dv.clear, s);
         dv.tri_wide = sc->tri_wide.as<float4>();
         dv.tri_wide_root = wt.root;
         dv.edge_wide = sc->edge_wide.as<float4>();
@@ -1199,7 +1289,7 @@ static TaskQueue task_queue(rtcd_detector* d, bool clear, cudaStream_t s, uint32
         cuda_check(cudaMemsetAsync(d->share.as<uint8_t>() + 256, 0xFF, slots, s), "memset");
     }
     uint8_t *base = d->share.as<uint8_t>(), *ctl = d->ctl.as<uint8_t>();
-    if (clear) cuda_check(cudaMemsetAsync(ctl + kCtlLive, 0, kCtlBytes - kCtlLive, s), "memset");
+    if (clear) cuda_check(cudaMemsetAsync(ctl + kCtlLive, 0, kCtlLinks - kCtlLive, s), "memset");
     TaskQueue q{};
     q.queue = reinterpret_cast<unsigned long long*>(base);
     q.live = reinterpret_cast<uint32_t*>(ctl + kCtlLive);
@@ -1226,6 +1316,13 @@ static void traverse(rtcd_detector* d, bool r2o, bool first, const DiscreteArgs&
     if (!(flags & RTCD_CHECK_FUSED) && !lane_form && R.pair_refs) {
         QueryArgs Q{};
         Q.d = A;
+        if (!A.link_count) {  // k_cull's items
+            uint32_t* lengths = reinterpret_cast<uint32_t*>(d->ctl.as<uint8_t>() + kCtlLinks);
+            d->lists.ensure(4ull * n * L);
+            if (first) launch_split_lists(A.items, A.n_items, n, L, d->lists.as<uint32_t>(), lengths, s);
+            Q.d.items = d->lists.as<uint32_t>();
+            Q.d.link_count = lengths;
+        }
         Q.share = task_queue(d, plain || !first, s, &Q.d.work_counter);
         launch_query(r2o, R, d->scene->dev, Q, (uint64_t) n * (L - R.first_link), share, plain ? blocks : 0xFFFFFFFFu, s);
         if (ev_first) cuda_check(cudaEventRecord(ev_first, s), "event");
@@ -1289,20 +1386,32 @@ static void traverse(rtcd_detector* d, bool r2o, bool first, const DiscreteArgs&
 // first, so RobotToObs skips the poses it decided; with counts RobotToObs
 // first, its edge counts then ObsToRobot's hits added); with
 // RTCD_CHECK_CONTAINMENT the containment test runs over the poses left.
+// d_flags: the check takes k_prepare's path (one_launch_prepare), which writes
+// the flags itself; NULL otherwise.
 void discrete_pass(rtcd_detector* d, const float* d_q, uint32_t n, uint32_t* d_hit, uint32_t* d_counts,
-                   uint32_t* d_bits, uint32_t* d_contain, uint32_t flags, bool plain, cudaStream_t s) {
+                   uint32_t* d_bits, uint32_t* d_contain, uint8_t* d_flags, uint32_t flags, bool plain, cudaStream_t s) {
     RobotDev& R = d->robot->dev;
     const uint32_t L = R.n_links;
     const bool counts = (flags & RTCD_CHECK_COUNTS) != 0;
     const bool two_way = (flags & RTCD_CHECK_TWO_WAY) != 0;
     d->T.ensure(48ull * n * L);
-    d->mask.ensure((size_t) n * L);
     d->items.ensure(4ull * n * L);
     const bool timed = (flags & RTCD_CHECK_TIMING) && !plain;
     if (timed) cuda_check(cudaEventRecord(d->ev[0], s), "event");
-    launch_fk_poses(R.chain, d_q, n, d->T.as<float4>(), s);
-    if (timed) cuda_check(cudaEventRecord(d->ev[1], s), "event");
-    if (flags & RTCD_CHECK_NO_CULL) {
+    uint32_t* link_count = nullptr;
+    if (d_flags) {  // FK, cull and item lists in one launch
+        if (timed) cuda_check(cudaEventRecord(d->ev[1], s), "event");
+        link_count = reinterpret_cast<uint32_t*>(d->ctl.as<uint8_t>() + kCtlLinks);
+        launch_prepare(R, d->scene->dev, d_q, n, (flags & RTCD_CHECK_NO_CULL) != 0, d->T.as<float4>(), d_hit, d_flags,
+                       link_count, d->items.as<uint32_t>(), s);
+    } else {
+        d->mask.ensure((size_t) n * L);
+        launch_fk_poses(R.chain, d_q, n, d->T.as<float4>(), s);
+        if (timed) cuda_check(cudaEventRecord(d->ev[1], s), "event");
+    }
+    d->last_lists = link_count != nullptr;
+    if (link_count) {
+    } else if (flags & RTCD_CHECK_NO_CULL) {
         launch_all_items(R, n, d->items.as<uint32_t>(), d->count.as<uint32_t>(), s);
     } else {
         launch_cull(R, d->scene->dev, d->T.as<float4>(), n, d->mask.as<uint8_t>(), true, d->stats(),
@@ -1321,6 +1430,8 @@ void discrete_pass(rtcd_detector* d, const float* d_q, uint32_t n, uint32_t* d_h
     }
     DiscreteArgs A{};
     A.T = d->T.as<float4>();
+    A.link_count = link_count;
+    A.flags = d_flags;
     A.items = d->items.as<uint32_t>();
     A.link_major = 1u;
     A.n_items = d->count.as<uint32_t>();
@@ -1354,6 +1465,14 @@ void discrete_pass(rtcd_detector* d, const float* d_q, uint32_t n, uint32_t* d_h
     d->timed = timed;
 }
 
+// Whether a check's FK, cull and flags are k_prepare's and the query kernel's: every batched check
+// of the query kernel, except that containment needs the items whose OBB reaches an obstacle's (a
+// link inside an obstacle touches none of its triangles).
+static bool one_launch_prepare(const rtcd_detector* d, uint32_t flags) {
+    return !(flags & (RTCD_CHECK_PLAIN | RTCD_CHECK_FUSED | RTCD_CHECK_CONTAINMENT)) && d->cfg.stage_b_form != 1 &&
+           d->cfg.stage_b_form != 2 && d->robot->dev.pair_refs && d->scene->dev.clear.gap;
+}
+
 void check_discrete(rtcd_detector* d, const float* q, uint32_t n, uint8_t* flags_out, uint32_t* counts_out,
                     uint32_t flags, cudaStream_t s) {
     const bool host = (flags & RTCD_CHECK_HOST_BUFFERS) != 0;
@@ -1372,8 +1491,14 @@ void check_discrete(rtcd_detector* d, const float* q, uint32_t n, uint8_t* flags
         cuda_check(cudaMemcpyAsync(d->q.p, src, 4ull * n * dof, cudaMemcpyHostToDevice, s), "q upload");
         d_q = d->q.as<float>();
     }
+    uint8_t* d_flags = flags_out;
+    if (host || !flags_out) {
+        d->flags.ensure(n);
+        d_flags = d->flags.as<uint8_t>();
+    }
+    const bool one = one_launch_prepare(d, flags);
     d->pose_hit.ensure(4ull * n);
-    cuda_check(cudaMemsetAsync(d->pose_hit.p, 0, 4ull * n, s), "memset");
+    if (!one) cuda_check(cudaMemsetAsync(d->pose_hit.p, 0, 4ull * n, s), "memset");
     uint32_t* d_counts = nullptr;
     uint32_t* d_bits = nullptr;
     uint32_t words = (R.n_edges_total + 31) / 32;
@@ -1431,7 +1556,7 @@ void check_discrete(rtcd_detector* d, const float* q, uint32_t n, uint8_t* flags
                     c->last_items = 0;
                     discrete_pass(c, d_q + (size_t) a * dof, m, d->pose_hit.as<uint32_t>() + a,
                                   d_counts ? d_counts + a : nullptr, d_bits ? d_bits + (size_t) a * words : nullptr,
-                                  d_contain ? d_contain + a : nullptr, flags, true, c->stream);
+                                  d_contain ? d_contain + a : nullptr, nullptr, flags, true, c->stream);
                 };
             }
             d->plain_pool->run(jobs);
@@ -1442,14 +1567,10 @@ void check_discrete(rtcd_detector* d, const float* q, uint32_t n, uint8_t* flags
             }
         }
     } else {
-        discrete_pass(d, d_q, n, d->pose_hit.as<uint32_t>(), d_counts, d_bits, d_contain, flags, false, s);
+        discrete_pass(d, d_q, n, d->pose_hit.as<uint32_t>(), d_counts, d_bits, d_contain, one ? d_flags : nullptr, flags,
+                      false, s);
     }
-    uint8_t* d_flags = flags_out;
-    if (host || !flags_out) {
-        d->flags.ensure(n);
-        d_flags = d->flags.as<uint8_t>();
-    }
-    launch_flags(d->pose_hit.as<uint32_t>(), n, d_flags, s, d_contain);
+    if (!one) launch_flags(d->pose_hit.as<uint32_t>(), n, d_flags, s, d_contain);
     if (host) {
         d->pin_out.ensure(5ull * n + 16);
         uint8_t* pf = d->pin_out.as<uint8_t>();
@@ -1838,7 +1959,12 @@ rtcd_status rtcd_last_stats(rtcd_detector* d, rtcd_stats* out) {
         uint32_t cnt = 0;
         cudaStream_t s = d->last_stream ? d->last_stream : d->stream;
         cuda_check(cudaMemcpyAsync(sb, d->stats(), sizeof(sb), cudaMemcpyDeviceToHost, s), "stats");
-        cuda_check(cudaMemcpyAsync(&cnt, d->count.p, 4, cudaMemcpyDeviceToHost, s), "stats");
+        uint32_t lists[kMaxLinks] = {0};
+        if (d->last_lists)
+            cuda_check(cudaMemcpyAsync(lists, d->ctl.as<uint8_t>() + kCtlLinks, sizeof(lists), cudaMemcpyDeviceToHost, s),
+                       "stats");
+        else
+            cuda_check(cudaMemcpyAsync(&cnt, d->count.p, 4, cudaMemcpyDeviceToHost, s), "stats");
         const bool discrete = d->kind == RTCD_OBS_TO_ROBOT || d->kind == RTCD_ROBOT_TO_OBS;
         uint32_t cand = 0, wave[4] = {0, 0, 0, 0}, work[2] = {0, 0};
         if (d->wave_counts.p)
@@ -1846,6 +1972,7 @@ rtcd_status rtcd_last_stats(rtcd_detector* d, rtcd_stats* out) {
         if (!discrete)
             cuda_check(cudaMemcpyAsync(work, d->work(), sizeof(work), cudaMemcpyDeviceToHost, s), "stats");
         cuda_check(cudaStreamSynchronize(s), "stats sync");
+        for (uint32_t c : lists) cnt += c;
         cand = wave[0];
         // the heavy list's append counter: [3] of the discrete wave counters, [1] of the sweep work words
         out->deferred = discrete ? wave[3] : work[1];

@@ -1,0 +1,107 @@
+// clearance.cu - the scene's clearance grid, read by the cull of k_prepare
+// (discrete.cu): for each cell of a grid over the scene's box a lower bound of
+// the distance from any point of the cell to the nearest triangle.
+//
+// Cells that a triangle touches are marked; the distance between two cells'
+// boxes is the root of the sum of their squared gaps along the axes, so three
+// passes, one per axis, give every cell the gap to its nearest marked cell
+// (a minimum over a line of cells of a value plus a squared gap; the usual
+// separable distance transform).
+#include <algorithm>
+#include <cmath>
+
+#include "kernels.h"
+
+namespace rtcd {
+
+constexpr int kClearCells = 256;   // cells along the scene's longest side
+constexpr int kClearReach = 63;    // cells; a larger gap counts as this one
+constexpr uint16_t kFar = kClearReach * kClearReach;
+
+// Cells are marked from each triangle's box, grown by 1e-5 m, where the
+// triangle's plane passes within a hundredth of a cell of the cell.
+__global__ void k_clear_mark(const float* __restrict__ v, const uint32_t* __restrict__ tris, uint32_t n, ClearGrid g,
+                             uint16_t* __restrict__ cells) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float *a = v + 3ull * tris[3ull * i], *b = v + 3ull * tris[3ull * i + 1], *c = v + 3ull * tris[3ull * i + 2];
+    int lo[3], hi[3];
+    for (int k = 0; k < 3; ++k) {
+        const float l = fminf(a[k], fminf(b[k], c[k])), h = fmaxf(a[k], fmaxf(b[k], c[k]));
+        lo[k] = clear_cell(g, k, l - 1e-5f);
+        hi[k] = clear_cell(g, k, h + 1e-5f);
+    }
+    const float size = 1.0f / g.inv;
+    const f3 p = mk(a[0], a[1], a[2]);
+    const f3 n3 = cross(mk(b[0], b[1], b[2]) - p, mk(c[0], c[1], c[2]) - p);
+    const float m = fabsf(n3.x) + fabsf(n3.y) + fabsf(n3.z), reach = (0.51f * size + 1e-5f) * m;
+    for (int z = lo[2]; z <= hi[2]; ++z)
+        for (int y = lo[1]; y <= hi[1]; ++y)
+            for (int x = lo[0]; x <= hi[0]; ++x) {
+                const f3 d = mk(g.org[0] + (x + 0.5f) * size, g.org[1] + (y + 0.5f) * size, g.org[2] + (z + 0.5f) * size) - p;
+                if (!(fabsf(dot(n3, d)) > reach)) cells[clear_at(g, x, y, z)] = 0;
+            }
+}
+
+// One pass: out = min over the cells j of the line along `axis`, within kClearReach, of in[j] plus
+// the squared gap between the two cells (in cells).
+__global__ void k_clear_pass(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, ClearGrid g, int axis) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+    if (x >= g.dim[0]) return;
+    const int at[3] = {x, y, z};
+    const int i = at[axis], n = g.dim[axis];
+    const long long step = axis == 0 ? 1 : axis == 1 ? g.dim[0] : (long long) g.dim[0] * g.dim[1];
+    const size_t here = clear_at(g, x, y, z);
+    uint32_t best = in[here];
+    for (int d = 1; d <= kClearReach; ++d) {
+        const uint32_t gap2 = (uint32_t) (d - 1) * (uint32_t) (d - 1);
+        if (gap2 >= best) break;
+        if (i - d >= 0) best = min(best, gap2 + in[here - d * step]);
+        if (i + d < n) best = min(best, gap2 + in[here + d * step]);
+    }
+    out[here] = (uint16_t) min(best, (uint32_t) kFar);
+}
+
+// Quarter cells, rounded down.
+__global__ void k_clear_pack(const uint16_t* __restrict__ in, uint8_t* __restrict__ out, size_t n) {
+    const size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x;
+    if (i < n) out[i] = (uint8_t) floorf(4.0f * sqrtf((float) in[i]) * 0.99999f);
+}
+
+bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tris, const float* lo, const float* hi,
+                     DevBuf& out, ClearGrid& g, cudaStream_t s) {
+    g = ClearGrid{};
+    if (!n_tris) return false;
+    const float pad = 1e-3f;
+    float longest = 0.f;
+    for (int k = 0; k < 3; ++k) {
+        const float extent = hi[k] - lo[k] + 2 * pad;
+        if (!(extent < 1e6f) || !(lo[k] > -1e6f)) return false;  // not finite, or cells beyond any use
+        longest = std::max(longest, extent);
+        g.org[k] = lo[k] - pad;
+    }
+    g.inv = (float) kClearCells / longest;
+    size_t cells = 1;
+    for (int k = 0; k < 3; ++k) {
+        g.dim[k] = std::min(kClearCells, std::max(1, (int) std::ceil((hi[k] - lo[k] + 2 * pad) * g.inv)));
+        cells *= (size_t) g.dim[k];
+    }
+    DevBuf a, b;
+    a.ensure(2 * cells);
+    b.ensure(2 * cells);
+    out.ensure(cells);
+    static_assert(0x1010 > kFar, "an unmarked cell starts beyond the cap");
+    cuda_check(cudaMemsetAsync(a.p, 0x10, 2 * cells, s), "clearance memset");
+    k_clear_mark<<<(n_tris + 127) / 128, 128, 0, s>>>(d_verts, d_tris, n_tris, g, a.as<uint16_t>());
+    const dim3 grid((g.dim[0] + 127) / 128, g.dim[1], g.dim[2]);
+    k_clear_pass<<<grid, 128, 0, s>>>(a.as<uint16_t>(), b.as<uint16_t>(), g, 0);
+    k_clear_pass<<<grid, 128, 0, s>>>(b.as<uint16_t>(), a.as<uint16_t>(), g, 1);
+    k_clear_pass<<<grid, 128, 0, s>>>(a.as<uint16_t>(), b.as<uint16_t>(), g, 2);
+    k_clear_pack<<<(uint32_t) ((cells + 255) / 256), 256, 0, s>>>(b.as<uint16_t>(), out.as<uint8_t>(), cells);
+    cuda_check(cudaGetLastError(), "clearance grid");
+    cuda_check(cudaStreamSynchronize(s), "clearance grid");  // the passes' buffers are released on return
+    g.gap = out.as<uint8_t>();
+    return true;
+}
+
+}  // namespace rtcd

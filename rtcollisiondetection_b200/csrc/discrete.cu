@@ -138,6 +138,89 @@ __device__ __forceinline__ uint32_t item_word(const DiscreteArgs& A, uint32_t n_
     return pose * n_links + link_slot(slot, n_links);
 }
 
+// FK, cull and item lists of a check that the query kernel answers: a block per
+// 32 poses, a warp per checked link.  Each warp runs the chain up to its link
+// (the links' chains run side by side, which costs less than handing transforms
+// on), then looks up the clearance (clearance.cu) at the centres of the spheres
+// that cover the link's mesh: a link whose spheres are all clear touches no
+// triangle.  A sphere outside the grid is clear if its centre moved to the
+// grid's box is (every triangle lies in the box).  What is not finite is kept.
+// The kept items go to their link's list, a warp's with one atomic add, and only
+// their transforms are written.
+//
+// Bound by the latency of the chain and the look-ups.  The OBB of every link
+// against every obstacle's (k_cull) is bound by its scan and by the divergence
+// of its 15-axis tests: with 321 obstacles and 65,536 poses 157 us, with FK,
+// compaction and their clears 195; this 46.
+constexpr int kPreparePoses = 32;
+__global__ void __launch_bounds__(kPreparePoses * kMaxLinks) k_prepare(const RobotDev R, const ClearGrid g,
+                                                                       const float* __restrict__ q, uint32_t n, bool all,
+                                                                       float4* __restrict__ T, uint32_t* __restrict__ hit,
+                                                                       uint8_t* __restrict__ flags,
+                                                                       uint32_t* __restrict__ link_count,
+                                                                       uint32_t* __restrict__ items) {
+    const int lane = threadIdx.x & 31, link = (int) R.first_link + (threadIdx.x >> 5), dof = R.chain.dof;
+    const uint32_t pose = blockIdx.x * kPreparePoses + lane;
+    const bool live = pose < n;
+    if (threadIdx.x < 32 && live) {
+        hit[pose] = 0;
+        if (flags) flags[pose] = 0;
+    }
+    float M[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) M[k] = R.chain.base[k];
+    for (int j = 0; j < link; ++j) {
+        float sn, cs;
+        sincosf(live ? __ldg(q + (size_t) pose * dof + j) : 0.f, &sn, &cs);
+        float Lm[12], N[12];
+#pragma unroll
+        for (int k = 0; k < 12; ++k)
+            Lm[k] = cs * R.chain.cm[j * 12 + k] + sn * R.chain.sm[j * 12 + k] + R.chain.om[j * 12 + k];
+        affine_mul(M, Lm, N);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) M[k] = N[k];
+    }
+    const float4 rows[3] = {make_float4(M[0], M[1], M[2], M[3]), make_float4(M[4], M[5], M[6], M[7]),
+                            make_float4(M[8], M[9], M[10], M[11])};
+    bool keep = live && all;
+    if (!all) {
+        const uint32_t end = R.cover_off[link + 1];
+        const float cell = 0.25f / g.inv;
+        for (uint32_t k = R.cover_off[link]; k < end; k += 4) {
+            bool touch = false;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {  // four look-ups in flight
+                const float4 sp = __ldg(R.cover + min(k + u, end - 1));
+                const f3 c = xf(rows, f3of(sp));
+                const float gap = cell * (float) __ldg(g.gap + clear_at(g, clear_cell(g, 0, c.x), clear_cell(g, 1, c.y),
+                                                                        clear_cell(g, 2, c.z)));
+                touch |= !(gap > sp.w) || !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < 1e30f);
+            }
+            keep |= live && touch;
+            if (__all_sync(0xffffffffu, keep || !live)) break;
+        }
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, keep), slot = link_slot(link, dof + 1);
+    uint32_t base = 0;
+    if (lane == 0 && m) base = atomicAdd(link_count + slot, (uint32_t) __popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (keep) {
+        items[(size_t) slot * n + base + __popc(m & ((1u << lane) - 1u))] = pose;
+        float4* out = T + ((size_t) pose * (dof + 1) + link) * 3;
+        out[0] = rows[0];
+        out[1] = rows[1];
+        out[2] = rows[2];
+    }
+}
+
+void launch_prepare(const RobotDev& R, const SceneDev& S, const float* d_q, uint32_t n, bool all, float4* d_T,
+                    uint32_t* d_hit, uint8_t* d_flags, uint32_t* d_link_count, uint32_t* d_items, cudaStream_t s) {
+    if (!n) return;
+    k_prepare<<<(n + kPreparePoses - 1) / kPreparePoses, kPreparePoses * (R.n_links - R.first_link), 0, s>>>(
+        R, S.clear, d_q, n, all, d_T, d_hit, d_flags, d_link_count, d_items);
+    cuda_check(cudaGetLastError(), "k_prepare");
+}
+
 // One thread per (pose, link): the link OBB against every obstacle OBB, with a
 // bounding-sphere reject before the full test.
 __global__ void __launch_bounds__(256) k_cull(const RobotDev R, const float* __restrict__ sobb, uint32_t n_obs,
@@ -186,6 +269,29 @@ void launch_cull(const RobotDev& R, const SceneDev& S, const float4* d_T, uint32
     if (!total) return;
     k_cull<<<(total + 255) / 256, 256, 0, s>>>(R, S.obbs, S.n_obs, d_T, n, d_mask, link_major, d_stats);
     cuda_check(cudaGetLastError(), "k_cull");
+}
+
+// The compacted items of k_cull as k_prepare's lists: one block per link's slot.
+__global__ void k_split_lists(const uint32_t* __restrict__ items, const uint32_t* __restrict__ n_items, uint32_t n,
+                              uint32_t* __restrict__ lists, uint32_t* __restrict__ link_count) {
+    const uint32_t slot = blockIdx.x, total = *n_items;
+    auto first = [&](unsigned long long v) {  // items are in order: how many are below v
+        uint32_t lo = 0, hi = total;
+        while (lo < hi) {
+            const uint32_t m = lo + (hi - lo) / 2;
+            if (items[m] < v) lo = m + 1; else hi = m;
+        }
+        return lo;
+    };
+    const uint32_t a = first((unsigned long long) slot * n), b = first((unsigned long long) (slot + 1) * n);
+    for (uint32_t k = threadIdx.x; k < b - a; k += blockDim.x) lists[(size_t) slot * n + k] = items[a + k] - slot * n;
+    if (threadIdx.x == 0) link_count[slot] = b - a;
+}
+
+void launch_split_lists(const uint32_t* d_items, const uint32_t* d_n_items, uint32_t n, uint32_t n_links,
+                        uint32_t* d_lists, uint32_t* d_link_count, cudaStream_t s) {
+    k_split_lists<<<n_links, 256, 0, s>>>(d_items, d_n_items, n, d_lists, d_link_count);
+    cuda_check(cudaGetLastError(), "k_split_lists");
 }
 
 // Every item, in the link-major order of the culled list (item_word): the
@@ -1116,10 +1222,19 @@ struct QueryWarp {
     CandCols<R2O> cols;
 };
 
+// Item `it` of k_prepare's lists (out of line: its registers would weigh on the kernel's loop).
+__device__ __noinline__ uint32_t list_item(const uint32_t* __restrict__ items, uint32_t n_poses, uint32_t n_links,
+                                           uint32_t it, const uint32_t* s_start) {
+    uint32_t slot = 0;
+    while (it >= s_start[slot + 1]) ++slot;
+    return items[(size_t) slot * n_poses + (it - s_start[slot])] * n_links + link_slot(slot, n_links);
+}
+
 template <bool R2O, int PER_SM>
 __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotDev R, const SceneDev S, const QueryArgs Q) {
     __shared__ QueryWarp<R2O> s_warp[kQueryWarps];
     __shared__ volatile uint32_t s_live;
+    __shared__ uint32_t s_start[kMaxLinks + 1];
     const DiscreteArgs& A = Q.d;
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -1131,7 +1246,14 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
     const float4* __restrict__ lp = R2O ? R.edge_prims : R.tri_prims;
     const int reserve_a = (int) frontier_reserve(R2O ? S.tri_wide_depth : S.edge_wide_depth);
     const int reserve_b = (int) frontier_reserve(R2O ? R.edge_wide_depth : R.tri_wide_depth);
-    const uint32_t n_items = *A.n_items, warps = gridDim.x * kQueryWarps;
+    const uint32_t warps = gridDim.x * kQueryWarps;
+    if (threadIdx.x <= R.n_links) {  // the lists' starts, one after another
+        uint32_t before = 0;
+        for (uint32_t k = 0; k < threadIdx.x; ++k) before += __ldg(A.link_count + k);
+        s_start[threadIdx.x] = before;
+    }
+    __syncthreads();
+    const uint32_t n_items = s_start[R.n_links];
     const bool counting = A.want_counts != 0;
     // blocks beyond the items and the waiting warps have nothing to do
     if (blockIdx.x * kQueryWarps >= n_items + Q.share.most_waiting) return;
@@ -1150,15 +1272,18 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
             }
             first = kNone;
             if (it < n_items) {
-                task.x = item_word(A, R.n_links, A.items[it]);
+                task.x = list_item(A.items, A.n_poses, R.n_links, it, s_start);
                 if (n_items - it > warps) poll = 4;
             } else {
                 listed = false;
                 share_wait_live(&s_live);
             }
         }
-        if (!listed && !take_task(Q.share, task)) break;
-        const uint32_t item = task.x, pose = item / R.n_links, link = item - pose * R.n_links;
+        if (!listed) {
+            task = take_task(Q.share);
+            if (task.x == kNone) break;
+        }
+        const uint32_t item = task.x, pose = item / R.n_links;
         if (pose >= A.n_poses) {
             if (lane == 0) atomicOr(A.err, kErrRange);
             continue;
@@ -1167,12 +1292,14 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
         if (lane == 0 && !counting) decided = ld_flag(A.pose_hit + pose);
         unsigned long long queue = 0;
         if (lane == 0) queue = look(Q.share.queue);
-        const uint32_t lroot = R2O ? R.edge_wide_root[link] : R.tri_wide_root[link];
         {
+            const uint32_t link = item - pose * R.n_links;
             ObbW ob;
             f3 ext;
             item_box(R, A, pose, link, ob, ext);
-            if (__shfl_sync(0xffffffffu, decided, 0) || lroot == kNone) continue;
+            if (__shfl_sync(0xffffffffu, decided, 0) ||
+                (R2O ? R.edge_wide_root[link] : R.tri_wide_root[link]) == kNone)
+                continue;
             if (lane == 0) s.obb.put(ob, ext);
             __syncwarp();
         }
@@ -1194,7 +1321,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
         if (lane == 0) n_cand += nc;
         auto share = [&](int most) {  // hands up to `most` nodes of the scene frontier to waiting warps
             const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
-            if (want > 0 && most > 0) offer_tasks(Q.share, min(want, most), [&](uint32_t) { return item; }, 0xFFFFFFFFu, s.front, sp);
+            if (want > 0 && most > 0) sp = offer_tasks(Q.share, min(want, most), item, nullptr, 0xFFFFFFFFu, s.front, sp);
             if (lane == 0) queue = look(Q.share.queue);
         };
         while (true) {
@@ -1215,10 +1342,12 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
             nc -= take;
             int np = 0, nl = 0;
             {
+                const uint32_t link = item - pose * R.n_links;
+                const uint32_t lroot = R2O ? R.edge_wide_root[link] : R.tri_wide_root[link];
                 StageBCand C;
                 bool live = false;
                 if (lane < take) {
-                    const float4* tp = A.T + ((size_t) pose * R.n_links + link) * 3;
+                    const float4* tp = A.T + (size_t) item * 3;
                     C.T[0] = __ldg(tp); C.T[1] = __ldg(tp + 1); C.T[2] = __ldg(tp + 2);
                     live = cand_geometry<R2O>(R, S, link, s.cand[nc + lane], C);
                     if (live) s.cols.put(lane, C);
@@ -1266,7 +1395,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
                     int r = seg_tri_f32(p, q, a, b, t);
                     if (r == 2) {
                         atomicAdd(A.stats, 1ull);
-                        r = retest_f64<R2O>(A.T + ((size_t) pose * R.n_links + link) * 3, lp, li, wp,
+                        r = retest_f64<R2O>(A.T + (size_t) item * 3, lp, li, wp,
                                             __float_as_uint(s.cols.f[CandCols<R2O>::kFields - 1][c]))
                                 ? 1 : 0;
                     }
@@ -1288,6 +1417,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
             if (pose_hit && lane == 0) {
                 if (counting) A.pose_hit[pose] = 1u;
                 else atomicExch(A.pose_hit + pose, 1u);
+                if (A.flags) A.flags[pose] = 1u;
             }
             // a hit, or another warp's meanwhile, decides the pose
             if (!counting && (pose_hit || __shfl_sync(0xffffffffu, decided, 0))) break;

@@ -22,6 +22,8 @@ struct RobotDev {
     const float4* edge_wide;
     uint32_t edge_wide_root[kMaxLinks];
     uint32_t tri_wide_depth, edge_wide_depth;  // deepest wide node of any link
+    const float4* cover;            // spheres (link frame) that hold every triangle and edge of a link
+    uint32_t cover_off[kMaxLinks + 1];
     uint32_t pair_refs;             // nonzero when every link reference fits beside a candidate's tag
     float4 link_point[kMaxLinks];   // one vertex of each link mesh (link frame)
     const float4* spheres;          // local centre xyz, radius w
@@ -29,8 +31,25 @@ struct RobotDev {
     uint32_t n_spheres;
 };
 
+// The scene's clearance grid (clearance.cu): cubic cells.
+struct ClearGrid {
+    float org[3], inv;   // cell of a coordinate: floor((x - org) * inv)
+    int dim[3];
+    const uint8_t* gap;  // [z][y][x] quarter cells, at most the distance to the nearest triangle; NULL: no grid
+};
+__host__ __device__ inline size_t clear_at(const ClearGrid& g, int x, int y, int z) {
+    return ((size_t) z * g.dim[1] + y) * g.dim[0] + x;
+}
+// The cell of x along axis k, the grid's first or last one outside it.
+__device__ __forceinline__ int clear_cell(const ClearGrid& g, int k, float x) {
+    return (int) fminf(fmaxf((x - g.org[k]) * g.inv, 0.0f), (float) (g.dim[k] - 1));
+}
+bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tris, const float* lo, const float* hi,
+                     DevBuf& out, ClearGrid& g, cudaStream_t s);
+
 // Scene resident on the device.
 struct SceneDev {
+    ClearGrid clear;
     const float4* tri_nodes;
     const float4* tri_prims;
     uint32_t tri_root;
@@ -56,6 +75,10 @@ struct SceneDev {
 
 struct DiscreteArgs {
     const float4* T;           // [pose][link][3] link transforms
+    const uint32_t* link_count;  // k_prepare's lists: items[slot * n_poses ...] holds link_count[slot] poses of the
+                                 // slot's link; NULL: items is one list (n_items, item_word), which
+                                 // the query kernel does not read
+    uint8_t* flags;            // [pose] set with pose_hit, or NULL
     const uint32_t* items;     // compacted (pose * n_links + link); NULL = all links >= first_link
     uint32_t link_major;       // items hold (link order slot) * n_poses + pose instead (see item_word)
     const uint32_t* n_items;   // device count of items
@@ -136,6 +159,13 @@ uint32_t stage_b_blocks(bool robot_to_obs);
 uint32_t stage_b_max_blocks_per_sm(bool robot_to_obs, uint32_t threads);  // threads: 64, 128 or 256
 
 void launch_fk_poses(const Chain& ch, const float* d_q, uint32_t n, float4* d_T, cudaStream_t s);
+// The compacted items of launch_cull / launch_all_items as launch_prepare's lists.
+void launch_split_lists(const uint32_t* d_items, const uint32_t* d_n_items, uint32_t n, uint32_t n_links,
+                        uint32_t* d_lists, uint32_t* d_link_count, cudaStream_t s);
+// FK, cull and per-link item lists in one launch: transforms (of the items kept), pose_hit and
+// flags zeroed, link_count (zeroed before) and items filled.  all: no cull.
+void launch_prepare(const RobotDev& R, const SceneDev& S, const float* d_q, uint32_t n, bool all, float4* d_T,
+                    uint32_t* d_hit, uint8_t* d_flags, uint32_t* d_link_count, uint32_t* d_items, cudaStream_t s);
 // link_major: the mask (and so the compacted items) in link order, every pose's
 // last link before any pose's next-to-last one (item_word decodes it).
 void launch_cull(const RobotDev& R, const SceneDev& S, const float4* d_T, uint32_t n, uint8_t* d_mask, bool link_major,

@@ -15,6 +15,7 @@
 
 namespace rtcd {
 
+constexpr uint32_t kShareTagShift = 27;  // an entry's tag above its node (wide.cuh)
 constexpr int kSharePolls = 1 << 16;  // polls of a word before a wait gives up
 
 // A slot is two 64-bit words, each with the ticket (plus one) it was written
@@ -71,9 +72,12 @@ __device__ __forceinline__ void end_if_all_wait(const TaskQueue& Q) {
     }
 }
 
-// A task for an idle warp (all lanes call): (owner's word, node); false when it
-// is to leave: the launch is over, or enough warps wait already (Q.most_waiting).
-__device__ __forceinline__ bool take_task(const TaskQueue& Q, uint2& task) {
+// A task for an idle warp (all lanes call): (owner's word, node); (kNone, 0) when
+// it is to leave: the launch is over, or enough warps wait already
+// (Q.most_waiting).  Out of line, like everything a warp does seldom: its
+// registers would weigh on the traversal loops.
+static __device__ __noinline__ uint2 take_task(const TaskQueue Q) {
+    uint2 task = make_uint2(kNone, 0u);
     const int lane = threadIdx.x & 31;
     uint32_t t = 0, leave = 0;
     if (lane == 0) {
@@ -83,7 +87,7 @@ __device__ __forceinline__ bool take_task(const TaskQueue& Q, uint2& task) {
         end_if_all_wait(Q);
     }
     leave = __shfl_sync(0xffffffffu, leave, 0);
-    if (leave) return false;
+    if (leave) return task;
     uint32_t got = 0;
     if (lane == 0) {
         ulonglong2* slot = Q.slot + (t & (Q.slots - 1));
@@ -131,15 +135,16 @@ __device__ __forceinline__ bool take_task(const TaskQueue& Q, uint2& task) {
     }
     task.x = __shfl_sync(0xffffffffu, task.x, 0);
     task.y = __shfl_sync(0xffffffffu, task.y, 0);
-    return __shfl_sync(0xffffffffu, got, 0) != 0;
+    if (!__shfl_sync(0xffffffffu, got, 0)) task.x = kNone;
+    return task;
 }
 
 // Hands up to `most` (at most 32) of the oldest of the entries fr[0, sp) to waiting
-// warps, or to the next ones that will be idle: an entry's node is its low bits (mask), its owner's word
-// owner(entry), below kWaiting.
-template <class Owner>
-__device__ __forceinline__ void offer_tasks(const TaskQueue& Q, int most, const Owner& owner, uint32_t mask, uint32_t* fr,
-                                            int& sp) {
+// warps, or to the next ones that will be idle.  An entry's node is its low bits
+// (mask); its owner's word, below kWaiting, is owners[its tag] (the bits above
+// the mask), or `owner` for every entry when owners is NULL.  Returns the new sp.
+static __device__ __noinline__ int offer_tasks(const TaskQueue Q, int most, uint32_t owner, const uint32_t* owners, uint32_t mask,
+                                        uint32_t* fr, int sp) {
     const int lane = threadIdx.x & 31;
     // every warp may offer once on one sight of the same waiting warps, and all of it fits the slots
     const int give = min(min(most, 32), (int) (Q.slots / (gridDim.x * (blockDim.x / 32))));
@@ -150,7 +155,7 @@ __device__ __forceinline__ void offer_tasks(const TaskQueue& Q, int most, const 
     bool kept = false;
     if (lane < give) {
         entry = fr[lane];
-        kept = !serve(Q, t0 + lane, owner(entry), entry & mask);
+        kept = !serve(Q, t0 + lane, owners ? owners[entry >> kShareTagShift] : owner, entry & mask);
     }
     const uint32_t mkept = __ballot_sync(0xffffffffu, kept);
     const int back = __popc(mkept);
@@ -163,8 +168,8 @@ __device__ __forceinline__ void offer_tasks(const TaskQueue& Q, int most, const 
         __syncwarp();
     }
     if (kept) fr[__popc(mkept & ((1u << lane) - 1u))] = entry;
-    sp -= give - back;
     __syncwarp();
+    return sp - (give - back);
 }
 
 // The block counts as live before a warp of it can be idle (all threads call, at

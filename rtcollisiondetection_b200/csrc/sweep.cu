@@ -1150,7 +1150,8 @@ __global__ void __launch_bounds__(kRestWarps * 32, QUAD ? 3 : 5) k_sweep_rest(co
             }
         }
         if (!listed) {
-            if (!take_task(A.share, task)) break;
+            task = take_task(A.share);
+            if (task.x == kNone) break;
             if (lane > 0) task.x = kNone;
         }
         unsigned long long queue = 0;
@@ -1180,8 +1181,7 @@ __global__ void __launch_bounds__(kRestWarps * 32, QUAD ? 3 : 5) k_sweep_rest(co
                 if ((++tick & (QUAD ? 0 : 3)) == 0) {
                     const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
                     if (want > 0 && np > 1)
-                        offer_tasks(A.share, min(want, np >> 1), [&](uint32_t e) { return s.cols.rec[e >> kTagShift]; },
-                                    kTagRef, s.pairs, np);
+                        np = offer_tasks(A.share, min(want, np >> 1), 0u, s.cols.rec, kTagRef, s.pairs, np);
                     if (lane == 0) queue = look(A.share.queue);
                     if (!counting) {  // the flags read at the last look, and read again for the next
                         test.alive &= __ballot_sync(0xffffffffu, decided == 0);
