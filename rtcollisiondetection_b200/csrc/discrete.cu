@@ -185,16 +185,13 @@ __global__ void __launch_bounds__(kPreparePoses * kMaxLinks) k_prepare(const Rob
     bool keep = live && all;
     if (!all) {
         const uint32_t end = R.cover_off[link + 1];
-        const float cell = 0.25f / g.inv;
         for (uint32_t k = R.cover_off[link]; k < end; k += 4) {
             bool touch = false;
 #pragma unroll
             for (uint32_t u = 0; u < 4; ++u) {  // four look-ups in flight
                 const float4 sp = __ldg(R.cover + min(k + u, end - 1));
                 const f3 c = xf(rows, f3of(sp));
-                const float gap = cell * (float) __ldg(g.gap + clear_at(g, clear_cell(g, 0, c.x), clear_cell(g, 1, c.y),
-                                                                        clear_cell(g, 2, c.z)));
-                touch |= !(gap > sp.w) || !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < 1e30f);
+                touch |= !(clearance(g, c.x, c.y, c.z) > sp.w) || !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < 1e30f);
             }
             keep |= live && touch;
             if (__all_sync(0xffffffffu, keep || !live)) break;

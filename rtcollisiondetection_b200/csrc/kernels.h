@@ -44,6 +44,11 @@ __host__ __device__ inline size_t clear_at(const ClearGrid& g, int x, int y, int
 __device__ __forceinline__ int clear_cell(const ClearGrid& g, int k, float x) {
     return (int) fminf(fmaxf((x - g.org[k]) * g.inv, 0.0f), (float) (g.dim[k] - 1));
 }
+// A lower bound of the distance from (x, y, z) to the nearest triangle.  (A point outside the grid's
+// box, which holds every triangle, is no nearer to any than its nearest point of the box.)
+__device__ __forceinline__ float clearance(const ClearGrid& g, float x, float y, float z) {
+    return (0.25f / g.inv) * (float) __ldg(g.gap + clear_at(g, clear_cell(g, 0, x), clear_cell(g, 1, y), clear_cell(g, 2, z)));
+}
 bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tris, const float* lo, const float* hi,
                      DevBuf& out, ClearGrid& g, cudaStream_t s);
 

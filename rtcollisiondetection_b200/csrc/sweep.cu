@@ -393,6 +393,33 @@ __device__ __forceinline__ void make_cull(const SweepUnit& U, SweepCull& c) {
     }
 }
 
+// True when the scene's clearance grid shows that no triangle, so no edge, comes
+// within reach of the unit: the chord's capsule lies in the sphere around its
+// middle, or else in four spheres along it, and each is clear.  Most units are:
+// 4,096 linear trajectories test 29M boxes with it and 181M without, and the
+// light pass takes 427 us instead of 989; quadratic 20M and 85M.  The light
+// passes look at 32 units a warp at a time, so the look-ups run on all lanes
+// (lane by lane, as units are needed, 10 of 32: 626 us).
+template <bool QUAD>
+__device__ __forceinline__ bool unit_clear(const ClearGrid& g, const SweepUnit& U, const SweepCull& c) {
+    if (!g.gap) return false;
+    const float4 Pe = QUAD ? U.P2 : U.P1;
+    const float dx = Pe.x - U.P0.x, dy = Pe.y - U.P0.y, dz = Pe.z - U.P0.z;
+    const float len = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f, reach = c.fat + 1e-4f;
+    // one copy of the look-up: the middle, then the four
+    bool clear = true;
+#pragma unroll 1
+    for (int k = 0; k < 5 && clear; ++k) {
+        const float t = k == 0 ? 0.5f : 0.25f * (float) k - 0.125f;
+        clear = clearance(g, U.P0.x + t * dx, U.P0.y + t * dy, U.P0.z + t * dz) > (k == 0 ? 0.5f : 0.125f) * len + reach;
+        if (k == 0) {
+            if (clear) return true;
+            clear = true;
+        }
+    }
+    return clear;
+}
+
 // t_enter: the chord parameter where it enters the grown box (visit order).
 template <bool QUAD>
 __device__ __forceinline__ bool cull_box(const SweepCull& c, const Box& b, float& t_enter) {
@@ -736,35 +763,71 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
     SweepUnit U;
     SweepCull c;
     U.traj = U.piece_g = 0;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t next = blockIdx.x * blockDim.x + threadIdx.x;  // neighbouring lanes: spheres of one piece
+    __shared__ uint32_t s_ready[BLOCK / 32][64];  // < 32 units waiting + 32 looked at together
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u, stride = gridDim.x * blockDim.x;
+    uint32_t* ready = s_ready[threadIdx.x >> 5];
+    uint32_t n_ready = 0;  // units near an obstacle that wait for a lane
+    uint64_t next = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);  // the warp's next 32: spheres of one piece or two
     unsigned long long n_acc = 0, n_skip = 0, n_leaf = 0, n_roots = 0, n_node = 0;
     const uint32_t budget = A.light_steps ? A.light_steps : 0xFFFFFFFFu;
 
     while (true) {
-        while (!busy && next < A.total_units) {
-            const uint32_t u = next;
-            next += stride;
-            if (!load_unit<QUAD>(A, u, U)) {
-                atomicOr(A.err, kErrRange);
-                continue;
+        // as in k_sweep_traj, with one copy of the set-up for both turns (the looked-at unit's and the
+        // handed-out one's): two copies are the faster there, one here
+        const uint32_t idle = __ballot_sync(0xffffffffu, !busy), n_idle = (uint32_t) __popc(idle);
+        bool more = next < A.total_units, look = n_idle > 0 && more && n_ready < n_idle;
+        while (look || (n_idle > 0 && n_ready > 0)) {
+            uint32_t u = A.total_units;
+            const uint32_t give = min(n_idle, n_ready), rank = (uint32_t) __popc(idle & lt);
+            if (look) {
+                if (next + lane < A.total_units) u = (uint32_t) next + lane;
+                next += stride;
+                more = next < A.total_units;
+            } else if (!busy && rank < give) {
+                u = ready[n_ready - 1 - rank];
             }
-            if (A.want_pieces ? ldflag(A.piece_hit + U.piece_g) && !A.want_counts
-                              : (!A.want_counts && ldflag(A.traj_hit + U.traj))) {
-                ++n_skip;
-                continue;
+            SweepUnit V;
+            SweepCull k;
+            bool near = false;
+            if (u < A.total_units) {
+                near = load_unit<QUAD>(A, u, V);
+                if (!near) atomicOr(A.err, kErrRange);
+                else if (!A.want_counts && ldflag(A.want_pieces ? A.piece_hit + V.piece_g : A.traj_hit + V.traj)) {
+                    ++n_skip;
+                    near = false;
+                }
+                near = near && root != kNone;
             }
-            if (root == kNone) continue;
-            make_cull<QUAD>(U, c);
-            st[0] = root;
-            sp = 1;
-            busy = true;
-            steps = 0;
-            checked = 0;
-            u_hits = 0;
-            ++n_acc;
+            if (near) make_cull<QUAD>(V, k);
+            if (!look) {
+                if (near) {
+                    U = V;
+                    c = k;
+                    st[0] = root;
+                    sp = 1;
+                    busy = true;
+                    steps = 0;
+                    checked = 0;
+                    u_hits = 0;
+                    ++n_acc;
+                }
+                n_ready -= give;
+                break;
+            }
+            if (near) near = !unit_clear<QUAD>(S.clear, V, k);
+            const uint32_t m = __ballot_sync(0xffffffffu, near);
+            if (near) ready[n_ready + __popc(m & lt)] = u;
+            n_ready += __popc(m);
+            __syncwarp();
+            look = more && n_ready < n_idle;
         }
-        if (!busy) break;
+        __syncwarp();
+        if (!__any_sync(0xffffffffu, busy)) {
+            if (!more && n_ready == 0) break;
+            continue;
+        }
+        if (!busy) continue;
         uint32_t leaf = kNone;
         // flags only: every 8 visits, drop a unit whose piece (or trajectory) another unit decided
         if (!A.want_counts && *decided == (A.want_pieces ? U.piece_g : U.traj)) sp = 0;
@@ -836,6 +899,7 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
     __shared__ uint32_t s_wb[kSweepMaxGroup + 1], s_ub[kSweepMaxGroup + 1], s_cb[kSweepMaxGroup + 1],
         s_pb[kSweepMaxGroup + 1];
     __shared__ volatile uint32_t s_hit[kSweepMaxGroup];
+    __shared__ uint32_t s_ready[BLOCK / 32][64];  // < 32 units waiting + 32 looked at together
     const float4* __restrict__ en = WIDE ? S.edge_wide : S.edge_nodes;
     const float4* __restrict__ ep = S.edge_prims;
     const uint32_t root = WIDE ? S.edge_wide_root : S.edge_root;
@@ -919,6 +983,51 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
             return make_float4(M[0] * p.x + M[1] * p.y + M[2] * p.z + M[3], M[4] * p.x + M[5] * p.y + M[6] * p.z + M[7],
                                M[8] * p.x + M[9] * p.y + M[10] * p.z + M[11], p.w);
         };
+        // unit u: its group member, piece and geometry; false when its piece (trajectory) is decided
+        auto setup = [&](uint32_t u, uint32_t& g, uint32_t& piece, SweepUnit& U) {
+            g = member(s_ub, u);
+            const uint32_t local = u - s_ub[g];
+            piece = local / ns;
+            const uint32_t s = local - piece * ns;
+            const volatile uint32_t* pf = reinterpret_cast<const volatile uint32_t*>(s_slots + (size_t) g * slot_words + f_at);
+            if (!A.want_counts && (A.want_pieces ? pf[piece] : s_hit[g])) {
+                ++n_skip;
+                return false;
+            }
+            const float* sT = s_slots + (size_t) g * slot_words;
+            const float4 sp4 = __ldg(R.spheres + s);
+            const uint32_t link = __ldg(R.sphere_link + s);
+            U.traj = s_tr0 + g;
+            U.piece_g = s_p0[g] + piece;
+            U.r = sp4.w;
+            if constexpr (!QUAD) {
+                U.P0 = at(sT + (size_t) (piece * L + link) * 12, sp4);
+                U.P1 = at(sT + (size_t) ((piece + 1) * L + link) * 12, sp4);
+                U.P2 = U.P1;
+            } else {
+                const uint32_t nc = (s_cb[g + 1] - s_cb[g]) / L12;
+                if (piece + 2 < nc) {
+                    const float* sC = sT + c_at;
+                    const float4 a = at(sC + (size_t) (piece * L + link) * 12, sp4);
+                    const float4 b = at(sC + (size_t) ((piece + 1) * L + link) * 12, sp4);
+                    const float4 cc = at(sC + (size_t) ((piece + 2) * L + link) * 12, sp4);
+                    U.P0 = make_float4(0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z), sp4.w);
+                    U.P1 = b;
+                    U.P2 = make_float4(0.5f * (b.x + cc.x), 0.5f * (b.y + cc.y), 0.5f * (b.z + cc.z), sp4.w);
+                } else {  // the start / end sphere
+                    const uint32_t w = (piece + 2 == nc) ? 0 : s_nwp[g] - 1;
+                    U.P0 = at(sT + (size_t) (w * L + link) * 12, sp4);
+                    U.P1 = U.P0;
+                    U.P2 = U.P0;
+                }
+            }
+            return root != kNone;
+        };
+        const int lane = threadIdx.x & 31;
+        const uint32_t lt = (1u << lane) - 1u;
+        uint32_t* ready = s_ready[threadIdx.x >> 5];
+        uint32_t n_ready = 0;  // units near an obstacle that wait for a lane
+        bool more = true;      // the group may hold more units
         int sp = 0;
         bool busy = false;
         uint32_t steps = 0, u_hits = 0, piece = 0, g = 0;
@@ -927,46 +1036,32 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
         U.traj = s_tr0;
         U.piece_g = 0;
         while (true) {
-            while (!busy) {
-                const uint32_t u = atomicAdd(&s_next, 1u);
-                if (u >= units) break;
-                g = member(s_ub, u);
-                const uint32_t local = u - s_ub[g];
-                piece = local / ns;
-                const uint32_t s = local - piece * ns;
-                const volatile uint32_t* pf = reinterpret_cast<const volatile uint32_t*>(s_slots + (size_t) g * slot_words + f_at);
-                if (!A.want_counts && (A.want_pieces ? pf[piece] : s_hit[g])) {
-                    ++n_skip;
-                    continue;
-                }
-                const float* sT = s_slots + (size_t) g * slot_words;
-                const float4 sp4 = __ldg(R.spheres + s);
-                const uint32_t link = __ldg(R.sphere_link + s);
-                U.traj = s_tr0 + g;
-                U.piece_g = s_p0[g] + piece;
-                U.r = sp4.w;
-                if constexpr (!QUAD) {
-                    U.P0 = at(sT + (size_t) (piece * L + link) * 12, sp4);
-                    U.P1 = at(sT + (size_t) ((piece + 1) * L + link) * 12, sp4);
-                    U.P2 = U.P1;
-                } else {
-                    const uint32_t nc = (s_cb[g + 1] - s_cb[g]) / L12;
-                    if (piece + 2 < nc) {
-                        const float* sC = sT + c_at;
-                        const float4 a = at(sC + (size_t) (piece * L + link) * 12, sp4);
-                        const float4 b = at(sC + (size_t) ((piece + 1) * L + link) * 12, sp4);
-                        const float4 cc = at(sC + (size_t) ((piece + 2) * L + link) * 12, sp4);
-                        U.P0 = make_float4(0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z), sp4.w);
-                        U.P1 = b;
-                        U.P2 = make_float4(0.5f * (b.x + cc.x), 0.5f * (b.y + cc.y), 0.5f * (b.z + cc.z), sp4.w);
-                    } else {  // the start / end sphere
-                        const uint32_t w = (piece + 2 == nc) ? 0 : s_nwp[g] - 1;
-                        U.P0 = at(sT + (size_t) (w * L + link) * 12, sp4);
-                        U.P1 = U.P0;
-                        U.P2 = U.P0;
+            const uint32_t idle = __ballot_sync(0xffffffffu, !busy), n_idle = (uint32_t) __popc(idle);
+            // the warp looks at 32 units at a time and keeps those that are not clear for its idle lanes
+            while (more && n_ready < n_idle) {
+                uint32_t u = 0;
+                if (lane == 0) u = atomicAdd(&s_next, 32u);
+                u = __shfl_sync(0xffffffffu, u, 0);
+                more = u + 32 < units;
+                u += lane;
+                bool near = false;
+                if (u < units) {
+                    SweepUnit V;
+                    SweepCull k;
+                    uint32_t vg, vp;
+                    near = setup(u, vg, vp, V);
+                    if (near) {
+                        make_cull<QUAD>(V, k);
+                        near = !unit_clear<QUAD>(S.clear, V, k);
                     }
                 }
-                if (root == kNone) continue;
+                const uint32_t m = __ballot_sync(0xffffffffu, near);
+                if (near) ready[n_ready + __popc(m & lt)] = u;
+                n_ready += __popc(m);
+                __syncwarp();
+            }
+            const uint32_t give = min(n_idle, n_ready), rank = (uint32_t) __popc(idle & lt);
+            if (!busy && rank < give && setup(ready[n_ready - 1 - rank], g, piece, U)) {
                 make_cull<QUAD>(U, c);
                 st[0] = root;
                 sp = 1;
@@ -975,7 +1070,13 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
                 u_hits = 0;
                 ++n_acc;
             }
-            if (!busy) break;
+            n_ready -= give;
+            __syncwarp();
+            if (!__any_sync(0xffffffffu, busy)) {
+                if (!more && n_ready == 0) break;
+                continue;
+            }
+            if (!busy) continue;
             volatile uint32_t* pf = reinterpret_cast<volatile uint32_t*>(s_slots + (size_t) g * slot_words + f_at);
             // flags only: drop the unit once its piece (or trajectory) is decided
             if (!A.want_counts && (A.want_pieces ? pf[piece] : s_hit[g])) sp = 0;
