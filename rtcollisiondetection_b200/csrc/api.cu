@@ -597,6 +597,7 @@ struct rtcd_detector {
     uint64_t graph_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     bool timed_total_only = false;       // the last check timed only ev[0] -> ev_end (graph path)
     uint32_t blocks = 0;
+    uint32_t staged_from = 0;  // trajectories from which the sweeps take the staged light pass
     // discrete workspace
     DevBuf q, T, mask, items, lists, count, pose_hit, counts, edge_bits, flags, seg_flags, err, ctl, contain;
     DevBuf share;  // the work sharing of a launch: counters and slots
@@ -663,7 +664,11 @@ static rtcd_status guarded(F&& f) {
 // Traversal launch shape from the detector config: threads per block (64, 128
 // or 256) and resident blocks per SM (0 or more than fit: as many as fit).
 static void apply_launch_shape(rtcd_detector* d) {
-    uint32_t t = d->cfg.traverse_threads ? d->cfg.traverse_threads : 128;
+    // 256 threads by default for the quadratic sweeps: a trajectory's long spline fit and its hand-over
+    // barrier are shared by twice the lanes (4,096 trajectories of 8-16 / 8-64 waypoints, cluttered scene,
+    // 532 -> 503 / 1,048 -> 1,002 us at 128 -> 256).  Linear trajectories have little to stage: 555 -> 629 us
+    // on 4,096 of 32 waypoints, so 128 stays there.
+    uint32_t t = d->cfg.traverse_threads ? d->cfg.traverse_threads : d->kind == RTCD_QUAD_SWEEP ? 256 : 128;
     if (t != 64 && t != 128 && t != 256) fail(RTCD_ERR_INVALID_ARGUMENT, "traverse_threads must be 64, 128 or 256");
     const bool discrete = d->kind == RTCD_OBS_TO_ROBOT || d->kind == RTCD_ROBOT_TO_OBS;
     uint32_t fit = discrete ? stage_b_max_blocks_per_sm(d->kind == RTCD_ROBOT_TO_OBS, t)
@@ -681,6 +686,15 @@ static void apply_launch_shape(rtcd_detector* d) {
         if (pct) d->blocks_a = std::max(sms, d->blocks_a_full * pct / 100);
     } else {
         d->blocks = per_sm * sms;
+        // The staged pass starts at four trajectories per resident block of 128 threads, whatever the kind:
+        // staged and unstaged splines round differently, so the line depends on the settings a caller gave only.
+        uint32_t rule = per_sm;
+        if (!d->cfg.traverse_threads && t != 128) {
+            fit = sweep_max_blocks_per_sm(d->kind == RTCD_QUAD_SWEEP, 128);
+            rule = d->cfg.traverse_blocks_per_sm ? std::min(d->cfg.traverse_blocks_per_sm, fit) : fit;
+            if (pct) rule = std::max(1u, rule * pct / 100);
+        }
+        d->staged_from = 4 * rule * sms;
     }
 }
 
@@ -1663,7 +1677,7 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
     // per resident block to keep the GPU busy: a batch of a few trajectories would run on a few
     // blocks (one trajectory of 128 waypoints is 8,128 units for one block) where the unstaged pass
     // spreads its units over the whole grid.
-    const bool staged = !d->cfg.sweep_unstaged && n >= 4 * d->blocks &&
+    const bool staged = !d->cfg.sweep_unstaged && n >= d->staged_from &&
                         sweep_staged_smem(quad, R.n_links, max_wp, max_nc, max_pieces) != 0;
     d->last_path_flags = staged ? 1u : 0u;
     const bool timed = (flags & RTCD_CHECK_TIMING) != 0;
@@ -1720,7 +1734,7 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
                                                               : 16u;
     A.descend_cap = d->cfg.sweep_descend_cap == 0xFFFFFFFFu ? 0u
                     : d->cfg.sweep_descend_cap                ? d->cfg.sweep_descend_cap
-                                                                  : 3u;
+                                                                  : (quad ? 2u : 3u);
     const SceneDev& scene = A.surface && A.total_units ? scene_loop(d->scene) : d->scene->dev;
     if (scene.n_edges >= (1u << 27)) A.light_steps = 0;  // the heavy pass holds an edge beside a column's tag (wide.cuh)
     if (A.light_steps) {
@@ -1742,7 +1756,12 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
         cuda_check(cudaEventRecord(d->ev[1], s), "event");
         cuda_check(cudaEventRecord(d->ev[2], s), "event");
     }
-    A.binary_tree = d->cfg.stage_b_form == 1 ? 1 : 0;
+    // The staged quadratic pass takes the binary tree by default: its loop is bound by instruction fetch
+    // (4.8 of 13 cycles per issue on the 4-wide form), and the binary step is the shorter code (4,096
+    // trajectories of 8-64 waypoints 1,184 -> 993 us, of 32 on a sparse scene 773 -> 769).  The unstaged
+    // lanes, few and latency-bound, keep the 4-wide tree (300 trajectories, sparse scene: 267 us against
+    // 338), and so do the linear sweeps (4,096 of 32 waypoints 555 us against 581).
+    A.binary_tree = d->cfg.stage_b_form == 1 || (d->cfg.stage_b_form == 0 && quad && staged) ? 1 : 0;
     if (A.total_units)
         launch_sweep(scene, R, A, d->blocks, d->threads,
                      d->cfg.residency_percent ? d->cfg.residency_percent : 100, staged, s,
@@ -2109,15 +2128,18 @@ rtcd_status rtcd_detector_autotune(rtcd_detector* d, const float* q_dev, const u
         auto form_pass = [&](const rtcd_config& base) {
             if (!discrete) {  // the binary or the wide edge tree, staged or unstaged centres, grouping
                 rtcd_config c = base;
-                c.stage_b_form = base.stage_b_form == 1 ? 0u : 1u;
-                time_cfg(c);
+                for (uint32_t form : {0u, 1u, 3u}) {  // 0: the default tree, 1: binary, 3: 4-wide
+                    if (form == base.stage_b_form) continue;
+                    c.stage_b_form = form;
+                    time_cfg(c);
+                }
                 c = base;
                 c.sweep_unstaged = base.sweep_unstaged ? 0u : 1u;
                 time_cfg(c);
                 c = base;
                 c.sweep_group = base.sweep_group == 1 ? 0u : 1u;
                 time_cfg(c);
-                for (uint32_t cap : {2u, 4u, 6u}) {  // visits per descent (0: the default, 3)
+                for (uint32_t cap : {2u, 3u, 4u, 6u}) {  // visits per descent (0: the kind's default, 2 or 3)
                     c = base;
                     c.sweep_descend_cap = base.sweep_descend_cap == cap ? 0u : cap;
                     time_cfg(c);
