@@ -823,8 +823,9 @@ def main():
         bytes_alg = n * (4 * model['cos_mask'].shape[0] + 1) + (64 + 48) * scene.n_tris + (64 + 32) * 35991
     achieved = bytes_alg / (t_trav / 1e3) / 1e9
     form = tuned.get('stage_b_form', 0)
+    dirs = 2 if args.two_way else 1
     if sweep:
-        span = ('k_sweep_traj' if st['path_flags'] & 1 else 'k_sweep') + ' + k_sweep_heavy x 2 (heavy, split)'
+        span = ('k_sweep_traj' if st['path_flags'] & 1 else 'k_sweep') + ' + k_sweep_rest'
     elif form in (0, 3, 4):
         span = 'k_query'
     else:
@@ -858,15 +859,16 @@ def main():
                 'frac': flops / (ms / 1e3) / 1e12 / FP32_PEAK_TFLOPS}
     kernels = {'traversal_span': kern(w_span, t_trav),
                'first_pass': dict(kern(w_first, t_first), kernel=span.split(' + ')[0] + ' (light pass)' if sweep else
-                                  ('k_stage_ab' if form in (0, 3, 4) else 'k_stage_a')),
+                                  ('k_query' if form in (0, 3, 4) else 'k_stage_a')),
                'later_passes': dict(kern(max(w_span - w_first, 0.0), t_rest),
-                                    kernel='k_sweep_heavy' if sweep else
-                                    'k_subtree x 2 + k_stage_b + k_stage_b_heavy + k_discrete')}
+                                    kernel='k_sweep_rest' if sweep else 'none' if form in (0, 3, 4) else
+                                    'k_stage_b + k_stage_b_heavy + k_discrete')}
     if not sweep:
         sats, sph = mean('cull_sat_tests'), mean('cull_sphere_tests')
         t_cull = float(np.mean([r['ms_cull'] for r in spans]))
         kernels['cull'] = dict(kern(180 * sats + 8 * sph + 36 * n * (links - 1), t_cull),
-                               kernel='k_cull + k_select_u8', sat_pairs=sats, sphere_tests=sph,
+                               kernel='k_prepare' if form in (0, 3, 4) and not args.containment
+                               else 'k_cull + k_select_u8', sat_pairs=sats, sphere_tests=sph,
                                all_pairs=n * (links - 1) * scene.n_obstacles)
     fp32 = {'achieved': kernels['traversal_span']['achieved'], 'peak': FP32_PEAK_TFLOPS, 'unit': 'TFLOP/s',
             'frac': kernels['traversal_span']['frac'], 'flops_per_step': w_span,
@@ -891,15 +893,14 @@ def main():
                    'launch_shape': tuned},
         'e2e': {'value': units_all / (e2e_step / 1e3), 'unit': unit, 'ms_per_step': e2e_step,
                 'h2d_bytes_per_step': int(h2d), 'd2h_bytes_per_step': int(d2h)},
-        # discrete: k_fk_poses, k_cull, k_select_u8, then per direction k_stage_ab + k_subtree x 2 + k_stage_b
-        # (deferred candidates) or k_stage_a + k_stage_b, k_stage_b_heavy, k_discrete (overflow); (k_contain),
-        # k_flags; sweeps: k_fk_spheres, (k_fit), k_sweep, k_sweep_heavy, k_flags x 2
-        # sweeps, staged light pass: k_sweep_traj, k_sweep_heavy, k_flags x 2; unstaged: k_fk_spheres, (k_fit),
-        # k_sweep, k_sweep_heavy, k_flags x 2
-        'gpu_launches': args.steps * ((3 + (2 if args.two_way else 1) * (6 if form in (0, 3, 4) else 4)
-                                       + (1 if args.containment else 0) + 1) if not sweep
-                                      # sweeps: light pass, heavy pass, its split pass, two flag gathers (+ FK and fit unstaged)
-                                      else 5 if st['path_flags'] & 1 else (6 if cfg['kind'] == 'Linear' else 7)),
+        # discrete, query kernel: k_prepare, then k_query per direction (it also writes the flags); with
+        # containment k_fk_poses, k_cull, k_select_u8, k_split_lists, k_query per direction, k_contain, k_flags;
+        # forms 1 and 2: k_fk_poses, k_cull, k_select_u8, per direction k_stage_a + k_stage_b + k_stage_b_heavy +
+        # k_discrete (overflow), (k_contain), k_flags.  Sweeps: k_sweep_traj, k_sweep_rest, k_sweep_flags; unstaged:
+        # k_fk_spheres, (k_fit), k_sweep, k_sweep_rest, k_sweep_flags
+        'gpu_launches': args.steps * (((1 + dirs if not args.containment else 6 + dirs) if form in (0, 3, 4)
+                                       else 3 + 4 * dirs + (1 if args.containment else 0) + 1) if not sweep
+                                      else 3 if st['path_flags'] & 1 else (4 if cfg['kind'] == 'Linear' else 5)),
         'stages_ms': {'prepare': float(np.mean([s['ms_prepare'] for s in spans])),
                       'cull': float(np.mean([s['ms_cull'] for s in spans])), 'traverse': t_trav},
         'roofline': {'bound': 'hbm', 'kernel': span, 'achieved': achieved,
