@@ -851,6 +851,8 @@ def main():
     if not sweep:
         cands = mean('candidates')
         w_span += 36 * cands   # every candidate primitive is moved into its link's frame
+        if form in (0, 3, 4):
+            w_first = w_span   # one kernel
     t_first = float(np.mean([r['ms_first_pass'] for r in spans]))
     t_rest = max(t_trav - t_first, 1e-6)
 
