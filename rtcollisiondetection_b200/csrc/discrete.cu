@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
         uint32_t decided = 0;
         if (lane == 0 && !counting) decided = ld_flag(A.pose_hit + pose);
         unsigned long long queue = 0;
-        if (lane == 0) queue = look(Q.share.queue);
+        if (lane == 0) queue = share_look(Q.share, &s_live);
         {
             const uint32_t link = item - pose * R.n_links;
             ObbW ob;
@@ -1319,7 +1319,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
         auto share = [&](int most) {  // hands up to `most` nodes of the scene frontier to waiting warps
             const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
             if (want > 0 && most > 0) sp = offer_tasks(Q.share, min(want, most), item, nullptr, 0xFFFFFFFFu, s.front, sp);
-            if (lane == 0) queue = look(Q.share.queue);
+            if (lane == 0) queue = share_look(Q.share, &s_live);
         };
         while (true) {
             if (nc < 32 && sp > 0) {  // stage A

@@ -123,8 +123,7 @@ struct WaveArgs {
 
 // Work sharing between the warps of a launch (share.cuh).
 struct TaskQueue {
-    unsigned long long* queue;  // low word: tickets taken by idle warps, high word: tasks offered; equal
-                                // between launches
+    unsigned long long* queue;  // tickets taken by idle warps, and tasks offered (share.cuh)
     uint32_t* live;             // warps of the blocks that have started; zeroed
     uint32_t* over;             // set once every live warp waits; zeroed
     uint32_t* err;              // device error word

@@ -6,10 +6,17 @@
 // to the waiting warps, one each.  The warp whose ticket makes every live warp a
 // waiting one ends all of them.  Live are the warps of the blocks that have
 // started: blocks still waiting for room beside another launch's are not waited
-// for, and find the list empty when they come.  A warp that finds enough others
-// waiting leaves.  A waiting warp gives up after a bounded time; what is offered
-// to a ticket that was given up stays with the warp that offered it, so no task
-// depends on a waiter.
+// for, and work through their own first entries after the end.  A warp that
+// finds enough others waiting leaves.  A waiting warp gives up after a bounded
+// time; what is offered to a ticket that was given up stays with the warp that
+// offered it.
+//
+// Offers follow a sight of the queue that is a step old, so a task may go to a
+// ticket that nobody has taken yet, before the end or after it.  No warp leaves
+// while more tasks are offered than tickets taken: the last one to have offered
+// looks after its offers, takes such a ticket and finds the task there.  So every
+// task runs, whatever the counts of live and waiting warps said meanwhile, and a
+// launch leaves no task behind for the next one.
 #pragma once
 #include "kernels.h"
 
@@ -25,8 +32,11 @@ constexpr int kSharePolls = 1 << 16;  // polls of a word before a wait gives up
 // ticket's warp (kWaiting) or the one that serves or ends the ticket, replaces
 // the first word once the slot's last ticket is done with it (free), the other
 // replaces the first one's; each with a compare-and-swap.  Tickets run on from
-// launch to launch, so slots are never cleared between them; the two counters
-// are added to as 32-bit words (no carry between them) and read as one.
+// launch to launch, so slots are never cleared between them.
+//
+// The queue word is read, added to and swapped as 64 bits: tickets taken in bits
+// 0 to 30, tasks offered in bits 32 to 62, both modulo 2^31.  Bit 31 takes the
+// carry of the first; whoever caused it clears it.
 constexpr uint32_t kTaken = 0xFFFFFFFFu, kGivenUp = 0xFFFFFFFEu, kWaiting = 0xFFFFFFFDu;
 __device__ __forceinline__ unsigned long long slot_word(uint32_t t, uint32_t v) {
     return ((unsigned long long) (t + 1) << 32) | v;
@@ -36,8 +46,11 @@ __device__ __forceinline__ unsigned long long look(const unsigned long long* p) 
     return *(const volatile unsigned long long*) p;
 }
 
+constexpr uint32_t kTicketMask = 0x7FFFFFFFu;
+__device__ __forceinline__ uint32_t taken(unsigned long long q) { return (uint32_t) q & kTicketMask; }
+__device__ __forceinline__ uint32_t offered(unsigned long long q) { return (uint32_t) (q >> 32) & kTicketMask; }
 // Tickets taken beyond the tasks offered: warps waiting for work.
-__device__ __forceinline__ int waiting(unsigned long long q) { return (int) ((uint32_t) q - (uint32_t) (q >> 32)); }
+__device__ __forceinline__ int waiting(unsigned long long q) { return (int) ((taken(q) - offered(q)) << 1) >> 1; }
 
 // Puts v into the slot of ticket t: false when its warp gave up.
 __device__ __forceinline__ bool serve(const TaskQueue& Q, uint32_t t, uint32_t v, uint32_t node) {
@@ -65,25 +78,35 @@ __device__ __forceinline__ void end_if_all_wait(const TaskQueue& Q) {
         const unsigned long long q = look(Q.queue);
         const int waits = waiting(q);
         if (waits < 0 || waits < (int) *(volatile uint32_t*) Q.live) return;
-        if (atomicCAS(Q.queue, q, (q << 32) | (uint32_t) q) == q) {
+        if (atomicCAS(Q.queue, q, ((unsigned long long) taken(q) << 32) | taken(q)) == q) {
             *(volatile uint32_t*) Q.over = 1u;
             return;
         }
     }
 }
 
+// A warp's leaving (one lane calls).  The last one checks that no task stays behind.
+__device__ __forceinline__ void leave_launch(const TaskQueue& Q) {
+    if (atomicSub(Q.live, 1u) == 1u && waiting(look(Q.queue)) < 0) atomicOr(Q.err, kErrLookback);
+}
+
 // A task for an idle warp (all lanes call): (owner's word, node); (kNone, 0) when
 // it is to leave: the launch is over, or enough warps wait already
-// (Q.most_waiting).  Out of line, like everything a warp does seldom: its
-// registers would weigh on the traversal loops.
+// (Q.most_waiting), and no task waits for a ticket.  Out of line, like everything
+// a warp does seldom: its registers would weigh on the traversal loops.
 static __device__ __noinline__ uint2 take_task(const TaskQueue Q) {
     uint2 task = make_uint2(kNone, 0u);
     const int lane = threadIdx.x & 31;
     uint32_t t = 0, leave = 0;
     if (lane == 0) {
-        leave = waiting(look(Q.queue)) >= (int) Q.most_waiting || *(volatile uint32_t*) Q.over;
-        if (leave) atomicSub(Q.live, 1u);
-        else t = atomicAdd(reinterpret_cast<uint32_t*>(Q.queue), 1u);
+        const int waits = waiting(look(Q.queue));
+        leave = waits >= (int) Q.most_waiting || (waits >= 0 && *(volatile uint32_t*) Q.over);
+        if (leave) {
+            leave_launch(Q);
+        } else {
+            t = taken(atomicAdd(Q.queue, 1ull));
+            if (t == kTicketMask) atomicAnd(Q.queue, ~(1ull << 31));
+        }
         end_if_all_wait(Q);
     }
     leave = __shfl_sync(0xffffffffu, leave, 0);
@@ -103,7 +126,7 @@ static __device__ __noinline__ uint2 take_task(const TaskQueue Q) {
                 if (gives_up) {  // unless a task arrives just now
                     if (atomicCAS(&slot->x, w, given) != w) continue;
                     w = given;
-                    atomicSub(Q.live, 1u);
+                    leave_launch(Q);
                     break;
                 }
                 if (w != wait) {  // first here
@@ -149,13 +172,13 @@ static __device__ __noinline__ int offer_tasks(const TaskQueue Q, int most, uint
     // every warp may offer once on one sight of the same waiting warps, and all of it fits the slots
     const int give = min(min(most, 32), (int) (Q.slots / (gridDim.x * (blockDim.x / 32))));
     uint32_t t0 = 0;
-    if (lane == 0) t0 = atomicAdd(reinterpret_cast<uint32_t*>(Q.queue) + 1, (uint32_t) give);
+    if (lane == 0) t0 = offered(atomicAdd(Q.queue, (unsigned long long) give << 32));
     t0 = __shfl_sync(0xffffffffu, t0, 0);
     uint32_t entry = 0;
     bool kept = false;
     if (lane < give) {
         entry = fr[lane];
-        kept = !serve(Q, t0 + lane, owners ? owners[entry >> kShareTagShift] : owner, entry & mask);
+        kept = !serve(Q, (t0 + lane) & kTicketMask, owners ? owners[entry >> kShareTagShift] : owner, entry & mask);
     }
     const uint32_t mkept = __ballot_sync(0xffffffffu, kept);
     const int back = __popc(mkept);
@@ -181,6 +204,10 @@ __device__ __forceinline__ void share_start(const TaskQueue& Q, volatile uint32_
 }
 __device__ __forceinline__ void share_wait_live(const volatile uint32_t* s_live) {
     for (int polls = 0; !*s_live && polls < kSharePolls; ++polls) {}
+}
+// A sight of the queue (one lane calls): no waiting warps until the block counts as live.
+__device__ __forceinline__ unsigned long long share_look(const TaskQueue& Q, const volatile uint32_t* s_live) {
+    return *s_live ? look(Q.queue) : 0ull;
 }
 
 }  // namespace rtcd

@@ -1256,7 +1256,7 @@ __global__ void __launch_bounds__(kRestWarps * 32, QUAD ? 3 : 5) k_sweep_rest(co
             if (lane > 0) task.x = kNone;
         }
         unsigned long long queue = 0;
-        if (lane == 0) queue = look(A.share.queue);
+        if (lane == 0) queue = share_look(A.share, &s_live);
         bool on = task.x != kNone;  // not a blank of a reservation that did not fit
         const uint32_t* flag = nullptr;
         uint32_t decided = 0;
@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(kRestWarps * 32, QUAD ? 3 : 5) k_sweep_rest(co
                     const int want = __shfl_sync(0xffffffffu, waiting(queue), 0);
                     if (want > 0 && np > 1)
                         np = offer_tasks(A.share, min(want, np >> 1), 0u, s.cols.rec, kTagRef, s.pairs, np);
-                    if (lane == 0) queue = look(A.share.queue);
+                    if (lane == 0) queue = share_look(A.share, &s_live);
                     if (!counting) {  // the flags read at the last look, and read again for the next
                         test.alive &= __ballot_sync(0xffffffffu, decided == 0);
                         if (on) decided = ldflag(flag);
