@@ -330,13 +330,14 @@ template <int DIM>
 static void launch_knn_dim(const float* pts, uint32_t n, const KnnWeights& w, uint32_t k, const uint8_t* mask,
                            uint32_t* idx, float* dist, cudaStream_t s) {
     constexpr size_t kMost = 200 * 1024;
+    constexpr size_t kStatic = 4 * 32 * (32 + DIM);  // k_knn's s_rank and s_q, part of a block's 48 KB without the opt-in
     const uint32_t blocks = (n + 31) / 32;
     uint32_t warps = 1;
     while (warps < 32 && 2 * warps <= blocks && (warps < 8 || blocks * warps < 16u * (uint32_t) device_sm_count()) &&
            2 * warps * knn_warp_bytes(k, DIM) <= kMost)
         warps *= 2;
     const size_t smem = warps * knn_warp_bytes(k, DIM);
-    if (smem > 47 * 1024)
+    if (smem + kStatic > 47 * 1024)
         cuda_check(cudaFuncSetAttribute(k_knn<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kMost), "k_knn");
     k_knn<DIM><<<blocks, warps * 32, smem, s>>>(pts, n, w, k, mask, idx, dist);
     cuda_check(cudaGetLastError(), "k_knn");
