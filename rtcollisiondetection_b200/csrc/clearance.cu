@@ -19,7 +19,11 @@ constexpr int kClearReach = 63;    // cells; a larger gap counts as this one
 constexpr uint16_t kFar = kClearReach * kClearReach;
 
 // Cells are marked from each triangle's box, grown by 1e-5 m, where the
-// triangle's plane passes within a hundredth of a cell of the cell.
+// triangle's plane passes within a hundredth of a cell of the cell.  In FP64: of
+// a sliver's FP32 normal little but rounding may be left, and a plane across it
+// leaves out cells that it passes through.  Corners on one line (to 1e-14 of the
+// sides) have no plane in FP64 either, and `rounding`, a bound of the normal's and the
+// product's errors, then lets every cell of the box through.
 __global__ void k_clear_mark(const float* __restrict__ v, const uint32_t* __restrict__ tris, uint32_t n, ClearGrid g,
                              uint16_t* __restrict__ cells) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -31,15 +35,15 @@ __global__ void k_clear_mark(const float* __restrict__ v, const uint32_t* __rest
         lo[k] = clear_cell(g, k, l - 1e-5f);
         hi[k] = clear_cell(g, k, h + 1e-5f);
     }
-    const float size = 1.0f / g.inv;
-    const f3 p = mk(a[0], a[1], a[2]);
-    const f3 n3 = cross(mk(b[0], b[1], b[2]) - p, mk(c[0], c[1], c[2]) - p);
-    const float m = fabsf(n3.x) + fabsf(n3.y) + fabsf(n3.z), reach = (0.51f * size + 1e-5f) * m;
+    const double size = 1.0 / g.inv;
+    const d3 p = dk(a[0], a[1], a[2]), e1 = dk(b[0], b[1], b[2]) - p, e2 = dk(c[0], c[1], c[2]) - p, n3 = cross(e1, e2);
+    const auto sum = [](d3 v) { return fabs(v.x) + fabs(v.y) + fabs(v.z); };
+    const double reach = (0.51 * size + 1e-5) * sum(n3), rounding = 1e-14 * sum(e1) * sum(e2);
     for (int z = lo[2]; z <= hi[2]; ++z)
         for (int y = lo[1]; y <= hi[1]; ++y)
             for (int x = lo[0]; x <= hi[0]; ++x) {
-                const f3 d = mk(g.org[0] + (x + 0.5f) * size, g.org[1] + (y + 0.5f) * size, g.org[2] + (z + 0.5f) * size) - p;
-                if (!(fabsf(dot(n3, d)) > reach)) cells[clear_at(g, x, y, z)] = 0;
+                const d3 d = dk(g.org[0] + (x + 0.5) * size, g.org[1] + (y + 0.5) * size, g.org[2] + (z + 0.5) * size) - p;
+                if (!(fabs(dot(n3, d)) > reach + rounding * sum(d))) cells[clear_at(g, x, y, z)] = 0;
             }
 }
 
