@@ -94,14 +94,18 @@ bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tr
     g = ClearGrid{};
     if (!n_tris) return false;
     const float pad = 1e-3f;
-    float longest = 0.f;
+    float longest = 0.f, most = 0.f;
     for (int k = 0; k < 3; ++k) {
         const float extent = hi[k] - lo[k] + 2 * pad;
         if (!(extent < 1e6f) || !(lo[k] > -1e6f)) return false;  // not finite, or cells beyond any use
         longest = std::max(longest, extent);
+        most = std::max({most, std::fabs(lo[k]), std::fabs(hi[k])});
         g.org[k] = lo[k] - pad;
     }
     g.inv = (float) kClearCells / longest;
+    // three axes, each with the rounding of a position (a bit of `most`) and of its cell (two of
+    // `longest`), with room: 5 um for a 3 m scene around the origin, 10 mm at 10 km from it
+    g.slack = 0x1p-20f * (most + longest);
     size_t cells = 1;
     for (int k = 0; k < 3; ++k) {
         g.dim[k] = std::min(kClearCells, std::max(1, (int) std::ceil((hi[k] - lo[k] + 2 * pad) * g.inv)));

@@ -34,6 +34,7 @@ struct RobotDev {
 // The scene's clearance grid (clearance.cu): cubic cells.
 struct ClearGrid {
     float org[3], inv;   // cell of a coordinate: floor((x - org) * inv)
+    float slack;         // what the rounding of positions may move a point or a cell's side
     int dim[3];
     const uint8_t* gap;  // [z][y][x] quarter cells, at most the distance to the nearest triangle; NULL: no grid
 };
@@ -47,7 +48,8 @@ __device__ __forceinline__ int clear_cell(const ClearGrid& g, int k, float x) {
 // A lower bound of the distance from (x, y, z) to the nearest triangle.  (A point outside the grid's
 // box, which holds every triangle, is no nearer to any than its nearest point of the box.)
 __device__ __forceinline__ float clearance(const ClearGrid& g, float x, float y, float z) {
-    return (0.25f / g.inv) * (float) __ldg(g.gap + clear_at(g, clear_cell(g, 0, x), clear_cell(g, 1, y), clear_cell(g, 2, z)));
+    return (0.25f / g.inv) * (float) __ldg(g.gap + clear_at(g, clear_cell(g, 0, x), clear_cell(g, 1, y), clear_cell(g, 2, z))) -
+           g.slack;
 }
 bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tris, const float* lo, const float* hi,
                      DevBuf& out, ClearGrid& g, cudaStream_t s);
