@@ -345,8 +345,10 @@ std::vector<uint32_t> loop_edges(const uint32_t* tris, size_t n_tris) {
 
 // Spheres that together hold every triangle and edge of a link, appended as
 // (centre, radius): its OBB is cut into about kCoverCells near-cubic cells, and
-// each cell with a primitive's centroid gets the sphere around the box of its
-// primitives' vertices (in the OBB's axes), grown by 1e-4 m.
+// each cell with a primitive's centroid gets a sphere about the middle of the box
+// of its primitives' vertices (in the OBB's axes), grown by 1e-4 m.  Radii are
+// taken in the link's frame: a caller's box need not hold the mesh, nor its axes
+// be of length 1 and at right angles.
 constexpr int kCoverCells = 24;
 
 static void cover_spheres(const float* verts, const uint32_t* tris, size_t n_tris, const uint32_t* edges, size_t n_edges,
@@ -358,7 +360,7 @@ static void cover_spheres(const float* verts, const uint32_t* tris, size_t n_tri
     for (int k = 0; k < 3; ++k) dim[k] = std::min(kCoverCells, std::max(1, (int) std::lround(2.0f * h[k] / size)));
     struct Cell {
         bool used = false;
-        float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f}, r2 = 0.f;
+        float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f}, mid[3] = {0, 0, 0}, r2 = 0.f;
     };
     std::vector<Cell> cells((size_t) dim[0] * dim[1] * dim[2]);
     auto local = [&](uint32_t v, float* x) {  // in the OBB's axes, from its centre
@@ -395,22 +397,22 @@ static void cover_spheres(const float* verts, const uint32_t* tris, size_t n_tri
             }
         }
     });
+    for (Cell& c : cells)
+        for (int a = 0; a < 3; ++a) {
+            c.mid[a] = obb[a];
+            for (int k = 0; k < 3; ++k) c.mid[a] += 0.5f * (c.lo[k] + c.hi[k]) * obb[6 + 3 * k + a];
+        }
     each([&](const uint32_t* idx, int m) {
         Cell& c = cell_of(idx, m);
         for (int j = 0; j < m; ++j) {
-            float x[3], r2 = 0.f;
-            local(idx[j], x);
-            for (int k = 0; k < 3; ++k) r2 += (x[k] - 0.5f * (c.lo[k] + c.hi[k])) * (x[k] - 0.5f * (c.lo[k] + c.hi[k]));
+            float r2 = 0.f;
+            for (int a = 0; a < 3; ++a) r2 += (verts[3ull * idx[j] + a] - c.mid[a]) * (verts[3ull * idx[j] + a] - c.mid[a]);
             c.r2 = std::max(c.r2, r2);
         }
     });
     for (const Cell& c : cells) {
         if (!c.used) continue;
-        for (int a = 0; a < 3; ++a) {
-            float v = obb[a];
-            for (int k = 0; k < 3; ++k) v += 0.5f * (c.lo[k] + c.hi[k]) * obb[6 + 3 * k + a];
-            out.push_back(v);
-        }
+        out.insert(out.end(), c.mid, c.mid + 3);
         out.push_back(std::sqrt(c.r2) * 1.0001f + 1e-4f);
     }
 }
