@@ -290,7 +290,8 @@ RTCD_API rtcd_status rtcd_sync(rtcd_detector* det, void* stream);
  * the binary and the 4-wide edge tree, staged or unstaged centres and
  * grouped or single trajectories; then the launch shapes again - rounds of
  * this coordinate descent until one changes nothing (at most three; sweeps
- * are timed with segment flags on)
+ * are timed with segment flags on; the query kernel takes no launch shape and
+ * no light budget, so it is timed once and reported with 128 threads)
  * - times each candidate's whole check replayed as a CUDA graph with device
  * events, after a write of twice the L2 size when free memory allows (median
  * of three replays after a warm-up run; the three fastest candidates are

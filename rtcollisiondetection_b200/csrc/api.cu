@@ -2106,7 +2106,22 @@ rtcd_status rtcd_detector_autotune(rtcd_detector* d, const float* q_dev, const u
         // coordinate descent: the launch shape, then the light-pass budget, then the stage B
         // form and its chunk length (discrete) or the tree and staging (sweeps), then the launch
         // shape again under the settings found (the best shape depends on them)
+        // (the query kernel takes neither a launch shape nor a light budget: it is timed once, and
+        // reported with its own 128 threads)
+        auto takes_shape = [&](const rtcd_config& c) {
+            return !discrete || c.stage_b_form == 1 || c.stage_b_form == 2 || !d->robot->dev.pair_refs;
+        };
+        auto time_query = [&] {
+            for (const auto& t : tried)
+                if (!takes_shape(t.second)) return;
+            rtcd_config c = saved;
+            c.stage_b_form = c.stage_b_chunk = 0;
+            c.traverse_threads = 128;
+            c.traverse_blocks_per_sm = stage_b_max_blocks_per_sm(d->kind == RTCD_ROBOT_TO_OBS, 128);
+            time_cfg(c);
+        };
         auto shape_pass = [&](const rtcd_config& base) {
+            if (!takes_shape(base)) return time_query();
             for (uint32_t t : {64u, 128u, 256u}) {
                 uint32_t fit = discrete ? stage_b_max_blocks_per_sm(d->kind == RTCD_ROBOT_TO_OBS, t)
                                         : sweep_max_blocks_per_sm(d->kind == RTCD_QUAD_SWEEP, t);
@@ -2121,6 +2136,7 @@ rtcd_status rtcd_detector_autotune(rtcd_detector* d, const float* q_dev, const u
             }
         };
         auto light_pass = [&](const rtcd_config& base) {
+            if (!takes_shape(base)) return;
             for (uint32_t light : {0u, 16u, 32u, 64u}) {  // 0: the kind's default budget
                 rtcd_config c = base;
                 c.light_steps = light;
@@ -2150,7 +2166,8 @@ rtcd_status rtcd_detector_autotune(rtcd_detector* d, const float* q_dev, const u
             }
             rtcd_config c = base;  // the query kernel, or the wavefront in lanes or packets
             c.stage_b_form = c.stage_b_chunk = 0;
-            time_cfg(c);
+            if (takes_shape(c)) time_cfg(c);
+            else time_query();
             for (uint32_t form : {1u, 2u})
                 for (uint32_t chunk : {1u, 16u, 64u, 256u}) {
                     c = base;
