@@ -1104,6 +1104,7 @@ void detector_info(rtcd_detector* d, rtcd_ctx** ctx, int* kind, rtcd_robot** rob
     *n_spheres = d->robot->dev.n_spheres;
     *dof = d->robot->dof;
 }
+uint32_t robot_edges(const rtcd_robot* robot) { return robot->dev.n_edges_total; }
 }  // namespace rtcd
 
 extern "C" {

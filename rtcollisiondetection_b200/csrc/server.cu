@@ -31,6 +31,7 @@
 namespace rtcd {
 void detector_info(rtcd_detector* d, rtcd_ctx** ctx, int* kind, rtcd_robot** robot, rtcd_scene** scene,
                    rtcd_config* cfg, uint32_t* n_links, uint32_t* n_spheres, uint32_t* dof);
+uint32_t robot_edges(const rtcd_robot* robot);
 }
 
 namespace {
@@ -95,11 +96,20 @@ struct rtcd_server {
 
 namespace {
 
-// Bytes a launch holds on the device (inputs, per-item state, candidate buffer).
-uint64_t estimate_bytes(int kind, uint64_t n, uint64_t units, uint32_t n_links, uint32_t n_spheres, uint32_t dof) {
-    if (!is_sweep(kind))
-        return n * (4ull * dof + 16) + n * n_links * (48ull + 1 + 4 + 1 + 4 + 8ull * 128);
-    return units * (4ull * dof + 2ull * 16 * n_spheres) + n * 16 + units * 8;
+// Bytes a launch holds on the device.  Discrete: inputs, results, and for each (pose, link) its
+// transform and list entries; with counts of link edges a row of bits per pose; in the wavefront
+// forms (stage_b_form 1 and 2) 128 candidates per (pose, link).  Sweeps: inputs, results and tables, the
+// spheres' centres and control points, and the lists of the heavy pass (a 64-byte record and four
+// 8-byte entries per (piece, sphere) unit, of at most 2^20 units).
+uint64_t estimate_bytes(int kind, const rtcd_config& cfg, uint64_t n, uint64_t units, uint32_t n_links, uint32_t n_spheres,
+                        uint32_t dof, uint32_t n_edges, bool counts) {
+    if (!is_sweep(kind)) {
+        const bool lanes = cfg.stage_b_form == 1 || cfg.stage_b_form == 2;
+        return n * (4ull * dof + 16) + n * n_links * (48ull + 1 + 4 + 4) +
+               (counts && kind == RTCD_ROBOT_TO_OBS ? n * (n_edges / 8 + 4) : 0) + (lanes ? n * n_links * (6ull + 8 * 128) : 0);
+    }
+    const uint64_t listed = cfg.light_steps == 0xFFFFFFFFu ? 0 : std::min<uint64_t>((units + 2 * n) * n_spheres, 1u << 20);
+    return units * (4ull * dof + 2ull * 16 * n_spheres) + n * 16 + units * 8 + listed * (64 + 4 * 8);
 }
 
 // The slot's clone of a user detector (created on first use).
@@ -199,7 +209,8 @@ void worker(rtcd_server* S, Slot* slot) {
             rtcd::detector_info(first->det, &c, &kind, &rb, &sc, &dc, &nl, &ns, &dof);
             uint64_t n = 0;
             for (Request* r : batch) n += r->n;
-            bytes = estimate_bytes(kind, n, units, nl, ns, dof);
+            bytes = estimate_bytes(kind, dc, n, units, nl, ns, dof, rtcd::robot_edges(rb),
+                                   (first->flags & RTCD_CHECK_COUNTS) != 0);
             S->cv_mem.wait(lk, [&] { return S->inflight_bytes == 0 || S->inflight_bytes + bytes <= S->cfg.memory_budget; });
             S->inflight_bytes += bytes;
             S->inflight_peak = std::max(S->inflight_peak, S->inflight_bytes);
