@@ -866,12 +866,16 @@ def main():
                                     kernel='k_sweep_rest' if sweep else 'none' if form in (0, 3, 4) else
                                     'k_stage_b + k_stage_b_heavy + k_discrete')}
     if not sweep:
-        sats, sph = mean('cull_sat_tests'), mean('cull_sphere_tests')
         t_cull = float(np.mean([r['ms_cull'] for r in spans]))
-        kernels['cull'] = dict(kern(180 * sats + 8 * sph + 36 * n * (links - 1), t_cull),
-                               kernel='k_prepare' if form in (0, 3, 4) and not args.containment
-                               else 'k_cull + k_select_u8', sat_pairs=sats, sphere_tests=sph,
-                               all_pairs=n * (links - 1) * scene.n_obstacles)
+        if form in (0, 3, 4) and not args.containment:
+            # one chain per checked link, of as many joints as come before it
+            kernels['cull'] = dict(kern(123 * n * links * (links - 1) / 2, t_cull), kernel='k_prepare',
+                                   counted='the chains; not the look-ups of covering spheres')
+        else:
+            sats, sph = mean('cull_sat_tests'), mean('cull_sphere_tests')
+            kernels['cull'] = dict(kern(180 * sats + 8 * sph + 36 * n * (links - 1), t_cull),
+                                   kernel='k_cull + k_select_u8', sat_pairs=sats, sphere_tests=sph,
+                                   all_pairs=n * (links - 1) * scene.n_obstacles)
     fp32 = {'achieved': kernels['traversal_span']['achieved'], 'peak': FP32_PEAK_TFLOPS, 'unit': 'TFLOP/s',
             'frac': kernels['traversal_span']['frac'], 'flops_per_step': w_span,
             'node_tests': nodes, 'leaf_tests': leaves, 'kernels': kernels,
@@ -879,7 +883,7 @@ def main():
                            '(148 SMs x 128 lanes x 2 x 1.965 GHz)',
             'weights': 'flops per counted op: node slab/box test 18, segment-triangle 40, segment-capsule 45, '
                        'segment-quadratic 200, candidate moved to the link frame 36, OBB SAT 180, '
-                       'bounding-sphere test 8, world OBB 36'}
+                       'bounding-sphere test 8, world OBB 36, joint of a chain 123'}
     if not args.no_check:
         fp32['reference_work'] = fp32_work(cfg, model, mesh, spheres, q, off, scene, t_trav)
     line = {
