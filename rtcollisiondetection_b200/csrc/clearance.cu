@@ -102,13 +102,13 @@ bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tr
         most = std::max({most, std::fabs(lo[k]), std::fabs(hi[k])});
         g.org[k] = lo[k] - pad;
     }
-    g.inv = (float) kClearCells / longest;
+    g.inv = (float) (kClearCells - 1) / longest;  // the triangles lie below the last cells' lower sides
     // three axes, each with the rounding of a position (a bit of `most`) and of its cell (two of
     // `longest`), with room: 5 um for a 3 m scene around the origin, 10 mm at 10 km from it
     g.slack = 0x1p-20f * (most + longest);
     size_t cells = 1;
     for (int k = 0; k < 3; ++k) {
-        g.dim[k] = std::min(kClearCells, std::max(1, (int) std::ceil((hi[k] - lo[k] + 2 * pad) * g.inv)));
+        g.dim[k] = std::min(kClearCells, 1 + std::max(1, (int) std::ceil((hi[k] - lo[k] + 2 * pad) * g.inv)));
         cells *= (size_t) g.dim[k];
     }
     DevBuf a, b;

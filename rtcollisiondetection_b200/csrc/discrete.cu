@@ -143,8 +143,7 @@ __device__ __forceinline__ uint32_t item_word(const DiscreteArgs& A, uint32_t n_
 // (the links' chains run side by side, which costs less than handing transforms
 // on), then looks up the clearance (clearance.cu) at the centres of the spheres
 // that cover the link's mesh: a link whose spheres are all clear touches no
-// triangle.  A sphere outside the grid is clear if its centre moved to the
-// grid's box is (every triangle lies in the box).  What is not finite is kept.
+// triangle.  What is not finite is kept.
 // The kept items go to their link's list, a warp's with one atomic add, and only
 // their transforms are written.
 //
@@ -191,7 +190,7 @@ __global__ void __launch_bounds__(kPreparePoses * kMaxLinks) k_prepare(const Rob
             for (uint32_t u = 0; u < 4; ++u) {  // four look-ups in flight
                 const float4 sp = __ldg(R.cover + min(k + u, end - 1));
                 const f3 c = xf(rows, f3of(sp));
-                touch |= !(clearance(g, c.x, c.y, c.z) > sp.w) || !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < 1e30f);
+                touch |= !clear_of(g, c.x, c.y, c.z, sp.w) || !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < 1e30f);
             }
             keep |= live && touch;
             if (__all_sync(0xffffffffu, keep || !live)) break;

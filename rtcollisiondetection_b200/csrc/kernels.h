@@ -45,11 +45,24 @@ __host__ __device__ inline size_t clear_at(const ClearGrid& g, int x, int y, int
 __device__ __forceinline__ int clear_cell(const ClearGrid& g, int k, float x) {
     return (int) fminf(fmaxf((x - g.org[k]) * g.inv, 0.0f), (float) (g.dim[k] - 1));
 }
-// A lower bound of the distance from (x, y, z) to the nearest triangle.  (A point outside the grid's
-// box, which holds every triangle, is no nearer to any than its nearest point of the box.)
-__device__ __forceinline__ float clearance(const ClearGrid& g, float x, float y, float z) {
-    return (0.25f / g.inv) * (float) __ldg(g.gap + clear_at(g, clear_cell(g, 0, x), clear_cell(g, 1, y), clear_cell(g, 2, z))) -
-           g.slack;
+// Whether every triangle is farther than r from (x, y, z).  The grid's points up to its last cells'
+// lower sides hold every triangle; with c the nearest one of them to p, a triangle's squared distance
+// from p is at least that from c, which the cell of c bounds, plus |p - c|^2.  Without the second term a
+// scene much smaller than the robot culls nothing: its whole grid is nearer than a link's spheres are wide.
+// False for what is not a number.
+__device__ __forceinline__ bool clear_of(const ClearGrid& g, float x, float y, float z, float r) {
+    const float at[3] = {x, y, z};
+    int cell[3];
+    float d2 = 0.0f;  // in cells
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float t = (at[k] - g.org[k]) * g.inv, c = fminf(fmaxf(t, 0.0f), (float) (g.dim[k] - 1));
+        cell[k] = (int) c;
+        d2 = fmaf(t - c, t - c, d2);
+    }
+    const float gap = 0.25f * (float) __ldg(g.gap + clear_at(g, cell[0], cell[1], cell[2]));
+    const float reach = (r + g.slack) * g.inv * 1.00001f;
+    return fmaf(gap, gap, d2) > reach * reach;
 }
 bool build_clearance(const float* d_verts, const uint32_t* d_tris, uint32_t n_tris, const float* lo, const float* hi,
                      DevBuf& out, ClearGrid& g, cudaStream_t s);

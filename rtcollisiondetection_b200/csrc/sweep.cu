@@ -411,7 +411,7 @@ __device__ __forceinline__ bool unit_clear(const ClearGrid& g, const SweepUnit& 
 #pragma unroll 1
     for (int k = 0; k < 5 && clear; ++k) {
         const float t = k == 0 ? 0.5f : 0.25f * (float) k - 0.125f;
-        clear = clearance(g, U.P0.x + t * dx, U.P0.y + t * dy, U.P0.z + t * dz) > (k == 0 ? 0.5f : 0.125f) * len + reach;
+        clear = clear_of(g, U.P0.x + t * dx, U.P0.y + t * dy, U.P0.z + t * dz, (k == 0 ? 0.5f : 0.125f) * len + reach);
         if (k == 0) {
             if (clear) return true;
             clear = true;
