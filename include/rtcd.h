@@ -127,9 +127,11 @@ typedef struct {
 typedef struct {
     uint32_t frame_size;             /* poses per frame of the plain path; 0 = 1024 (the upstream benchmark's
                                         batchSize, RTCD/Benchmark/Discrete/benchmarkUtils.h:16) */
-    uint32_t traverse_threads;       /* threads per block of the traversal kernel: 64, 128 or 256; 0 = 128,
-                                        256 for the quadratic sweeps */
-    uint32_t traverse_blocks_per_sm; /* resident traversal blocks per SM; 0 = as many as fit */
+    uint32_t traverse_threads;       /* threads per block of the sweeps' light pass and of the discrete forms 1 and 2
+                                        (stage_b_form): 64, 128 or 256; 0 = 128, 256 for quadratic sweeps with
+                                        segment flags or counts.  The query kernel has 128 whatever is given */
+    uint32_t traverse_blocks_per_sm; /* their resident blocks per SM; 0 = as many as fit.  Without effect on the query
+                                        kernel, which residency_percent limits */
     int32_t stream_priority;         /* priority of the detector's own stream (CUDA convention: lower = higher) */
     uint32_t residency_percent;      /* share of each SM its persistent kernels may hold (room for other
                                         launches to run alongside); 0 = 100 */
@@ -144,7 +146,8 @@ typedef struct {
                                         32-candidate packets that share each link-BVH node load.  Sweeps: 1 =
                                         the light pass's lanes descend the binary edge tree, 2 to 4 = the
                                         4-wide one (when the scene's is shallow enough for a lane stack),
-                                        0 = binary for the staged quadratic pass, 4-wide otherwise.
+                                        0 = binary for the staged quadratic pass (unless light_steps is
+                                        0xFFFFFFFF), 4-wide otherwise.
                                         The autotuner tries them */
     uint32_t stage_b_chunk;          /* discrete forms 1 and 2: consecutive candidates one lane takes in order (lanes
                                         form) or 32-candidate groups one warp takes (packets), so a pose's
@@ -171,8 +174,8 @@ typedef struct {
     uint32_t sweep_descend_cap;      /* sweeps, light pass: node visits a lane makes in one descent before the
                                         warp's lanes without work take new units (the descent then resumes
                                         where it stopped), so a lane that finished a short unit does not wait
-                                        out a long one; 0 = 3 (2 for the quadratic
-                                        sweeps), 0xFFFFFFFF = every descent runs to its next
+                                        out a long one; 0 = 3 (2 for the quadratic sweeps,
+                                        unless light_steps is 0xFFFFFFFF), 0xFFFFFFFF = every descent runs to its next
                                         leaf (the autotuner tries 2, 3, 4 and 6) */
     uint32_t sweep_heavy_wide;       /* accepted, without effect (the heavy pass descends the 4-wide edge tree) */
 } rtcd_config;

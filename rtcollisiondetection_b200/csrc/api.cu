@@ -663,14 +663,21 @@ static rtcd_status guarded(F&& f) {
         if (!(cond)) fail(RTCD_ERR_INVALID_ARGUMENT, msg); \
     } while (0)
 
+// Whether the quadratic sweeps' own defaults apply (the settings that are 0): they suit a light pass
+// that hands long units over.
+static bool quad_defaults(const rtcd_detector* d) {
+    return d->kind == RTCD_QUAD_SWEEP && d->cfg.light_steps != 0xFFFFFFFFu;
+}
+
 // Traversal launch shape from the detector config: threads per block (64, 128
 // or 256) and resident blocks per SM (0 or more than fit: as many as fit).
 static void apply_launch_shape(rtcd_detector* d) {
     // 256 threads by default for the quadratic sweeps: a trajectory's long spline fit and its hand-over
     // barrier are shared by twice the lanes (4,096 trajectories of 8-16 / 8-64 waypoints, cluttered scene,
-    // 532 -> 503 / 1,048 -> 1,002 us at 128 -> 256).  Linear trajectories have little to stage: 555 -> 629 us
-    // on 4,096 of 32 waypoints, so 128 stays there.
-    uint32_t t = d->cfg.traverse_threads ? d->cfg.traverse_threads : d->kind == RTCD_QUAD_SWEEP ? 256 : 128;
+    // 532 -> 503 / 1,048 -> 1,002 us at 128 -> 256; a sparse scene is the slower for it, 32 waypoints 715 ->
+    // 758).  Linear trajectories have little to stage: 555 -> 629 us on 4,096 of 32 waypoints, so 128 stays
+    // there, and so it does where the light pass hands nothing over (3,654 us against 4,300).
+    uint32_t t = d->cfg.traverse_threads ? d->cfg.traverse_threads : quad_defaults(d) ? 256 : 128;
     if (t != 64 && t != 128 && t != 256) fail(RTCD_ERR_INVALID_ARGUMENT, "traverse_threads must be 64, 128 or 256");
     const bool discrete = d->kind == RTCD_OBS_TO_ROBOT || d->kind == RTCD_ROBOT_TO_OBS;
     uint32_t fit = discrete ? stage_b_max_blocks_per_sm(d->kind == RTCD_ROBOT_TO_OBS, t)
@@ -1737,7 +1744,7 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
                                                               : 16u;
     A.descend_cap = d->cfg.sweep_descend_cap == 0xFFFFFFFFu ? 0u
                     : d->cfg.sweep_descend_cap                ? d->cfg.sweep_descend_cap
-                                                                  : (quad ? 2u : 3u);
+                                                                  : (quad_defaults(d) ? 2u : 3u);
     const SceneDev& scene = A.surface && A.total_units ? scene_loop(d->scene) : d->scene->dev;
     if (scene.n_edges >= (1u << 27)) A.light_steps = 0;  // the heavy pass holds an edge beside a column's tag (wide.cuh)
     if (A.light_steps) {
@@ -1764,9 +1771,19 @@ void check_sweep(rtcd_detector* d, const float* q, const uint32_t* traj_off, uin
     // trajectories of 8-64 waypoints 1,184 -> 993 us, of 32 on a sparse scene 773 -> 769).  The unstaged
     // lanes, few and latency-bound, keep the 4-wide tree (300 trajectories, sparse scene: 267 us against
     // 338), and so do the linear sweeps (4,096 of 32 waypoints 555 us against 581).
-    A.binary_tree = d->cfg.stage_b_form == 1 || (d->cfg.stage_b_form == 0 && quad && staged) ? 1 : 0;
+    A.binary_tree = d->cfg.stage_b_form == 1 || (d->cfg.stage_b_form == 0 && quad_defaults(d) && staged) ? 1 : 0;
+    uint32_t blocks = d->blocks, threads = d->threads;
+    // With neither segment flags nor counts a trajectory ends at its first hit, and the lanes of a larger
+    // block are idle then: 4,000 trajectories of 24 waypoints at 128 / 256 threads 235 / 309 us (a table),
+    // 369 / 506 and 463 / 572 (shelves), 445 / 597 (clutter), 310 / 456 (428k triangles).  With segment
+    // flags 816 / 836, 847 / 907, 585 / 614 on the last three: but 1,045 / 1,003, 884 / 826 and
+    // 827 / 791 on 4,096 of 8 to 64.
+    if (staged && quad_defaults(d) && !d->cfg.traverse_threads && !want_pieces && !counts) {
+        threads = 128;
+        blocks = d->staged_from / 4;
+    }
     if (A.total_units)
-        launch_sweep(scene, R, A, d->blocks, d->threads,
+        launch_sweep(scene, R, A, blocks, threads,
                      d->cfg.residency_percent ? d->cfg.residency_percent : 100, staged, s,
                      timed ? d->ev_first : nullptr);
     else if (timed)

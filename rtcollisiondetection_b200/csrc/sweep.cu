@@ -1028,6 +1028,12 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
         uint32_t* ready = s_ready[threadIdx.x >> 5];
         uint32_t n_ready = 0;  // units near an obstacle that wait for a lane
         bool more = true;      // the group may hold more units
+        // Without counts and segment flags a group ends with its trajectories' first hits: a warp stops
+        // looking when all have one, and looks less far ahead of its descents for them (linear, all hit by
+        // a table: 4,000 trajectories 191 -> 150 us, start of the descents at 8 units instead of 32;
+        // quadratic units are better collected, 452 us against 473 on 4,000 in clutter).
+        const bool flags_only = !A.want_counts && !A.want_pieces;
+        const uint32_t ahead = flags_only && !QUAD ? 8u : 32u;
         int sp = 0;
         bool busy = false;
         uint32_t steps = 0, u_hits = 0, piece = 0, g = 0;
@@ -1038,8 +1044,16 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
         while (true) {
             const uint32_t idle = __ballot_sync(0xffffffffu, !busy), n_idle = (uint32_t) __popc(idle);
             // the warp looks at 32 units at a time and keeps those that are not clear for its idle lanes
-            while (more && n_ready < n_idle) {
+            while (more && n_ready < min(n_idle, ahead)) {
                 uint32_t u = 0;
+                if (flags_only && __all_sync(0xffffffffu, lane >= s_ng || s_hit[lane & (kSweepMaxGroup - 1)])) {
+                    if (lane == 0) {
+                        u = atomicExch(&s_next, units);
+                        n_skip += units - min(u, units);
+                    }
+                    more = false;
+                    break;
+                }
                 if (lane == 0) u = atomicAdd(&s_next, 32u);
                 u = __shfl_sync(0xffffffffu, u, 0);
                 more = u + 32 < units;
