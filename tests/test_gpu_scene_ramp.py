@@ -30,3 +30,11 @@ def test_ramp_is_made_quickly(ctx, panda, ramp):
     b = _time(ctx, scenes.Mesh(small, np.array([[0, 1, 2], [3, 4, 5]]), np.array([0, 2])))
     print('ramp %.1f ms, the same grid without it %.1f ms' % (1e3 * a, 1e3 * b))
     assert a < b + 0.1
+
+
+def test_small_part_is_made_quickly(ctx, panda):
+    """The grid of a part of a few centimetres is small (0.4 ms without a grid, 4.7 with 256 cells along it)."""
+    v, t = scenes.box_mesh((0.5, 0.1, 0.4), (0.05, 0.03, 0.05))
+    a = min(_time(ctx, scenes.Mesh(v, t, np.array([0, len(t)]))) for _ in range(4))
+    print('small part %.2f ms' % (1e3 * a))
+    assert a < 0.002
