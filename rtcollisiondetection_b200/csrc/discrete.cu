@@ -150,7 +150,7 @@ __device__ __forceinline__ uint32_t item_word(const DiscreteArgs& A, uint32_t n_
 // Bound by the latency of the chain and the look-ups.  The OBB of every link
 // against every obstacle's (k_cull) is bound by its scan and by the divergence
 // of its 15-axis tests: with 321 obstacles and 65,536 poses 157 us, with FK,
-// compaction and their clears 195; this 46.
+// compaction and their clears 195; this 50.
 constexpr int kPreparePoses = 32;
 __global__ void __launch_bounds__(kPreparePoses * kMaxLinks) k_prepare(const RobotDev R, const ClearGrid g,
                                                                        const float* __restrict__ q, uint32_t n, bool all,
@@ -1439,7 +1439,8 @@ __global__ void __launch_bounds__(kQueryWarps * 32, PER_SM) k_query(const RobotD
 // blocks from leaving the SMs to other launches.  Whole checks of uniform poses at three / five blocks per SM, in us,
 // RobotToObs on the 428k-triangle scene: 4,096 poses 200 / 216, 8,192 253 / 263,
 // 16,384 397 / 373, 32,768 691 / 621; on the 202k-triangle shelf: 4,096 168 / 180,
-// 16,384 271 / 300, 32,768 393 / 395.
+// 16,384 271 / 300, 32,768 393 / 395.  So the two cross at 10,000 to 30,000 poses, by scene; the line, 16,237
+// poses on 148 SMs, costs either of these two a tenth at most.
 constexpr uint32_t kQueryFew = 768;
 template <bool R2O>
 static void query_dispatch(const RobotDev& R, const SceneDev& S, const QueryArgs& Q, uint64_t items, uint32_t share,

@@ -397,7 +397,7 @@ __device__ __forceinline__ void make_cull(const SweepUnit& U, SweepCull& c) {
 // within reach of the unit: the chord's capsule lies in the sphere around its
 // middle, or else in four spheres along it, and each is clear.  Most units are:
 // 4,096 linear trajectories test 29M boxes with it and 181M without, and the
-// light pass takes 427 us instead of 989; quadratic 20M and 85M.  The light
+// light pass takes 439 us instead of 989; quadratic 20M and 85M.  The light
 // passes look at 32 units a warp at a time, so the look-ups run on all lanes
 // (lane by lane, as units are needed, 10 of 32: 626 us).
 template <bool QUAD>
@@ -738,7 +738,7 @@ __device__ __forceinline__ bool hand_over(const SceneDev& S, const SweepArgs& A,
 // A.light_steps node and leaf visits is handed to the heavy pass (hand_over),
 // so one lane never serialises a unit that meets thousands of nodes.
 // The quadratic form is capped at 96 registers (5 blocks of 128 threads per
-// SM), the linear one at 80 (6 blocks): the extra resident warps hide more
+// SM; 2 of 256, capped at 128), the linear one at 80 (6 blocks): the extra resident warps hide more
 // load latency than the few spilled registers cost (measured on the
 // 4,096-trajectory workloads; 6 blocks slowed the quadratic form).
 // WIDE: the descent runs over the scene's 4-wide edge tree (a node's four
@@ -1149,9 +1149,9 @@ __global__ void __launch_bounds__(BLOCK, QUAD ? 5 * 128 / BLOCK : 6 * 128 / BLOC
 // A warp per unit from the root, and a second launch for the units it did not
 // finish in 32 steps, took 258 us for the 53k open units of 4,096 linear
 // trajectories, 452 us for 45k quadratic ones and 5.2 ms for the 24k of 301
-// trajectories counted over the 202k-triangle shelf; this 116 us, 302 us and
-// 2.3 ms.  Bound by the latency of node and edge loads and, counting, by the
-// 59M edges to test.  More than five (quadratic: three) blocks per SM are
+// trajectories counted over the 202k-triangle shelf; this 116 us, 302 us (374
+// from the root, as the binary light pass hands over) and 2.3 ms.  Bound by the
+// latency of node and edge loads and, counting, by the 59M edges to test.  More than five (quadratic: three) blocks per SM are
 // slower by up to 6 %.
 constexpr int kRestWarps = 4;
 constexpr int kRestPairs = 512;
